@@ -23,6 +23,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include "soft64.cuh"
 #include "sts_internal.cuh"
 
 struct StageArgs {
@@ -204,89 +205,67 @@ struct VecIO<float, 4> {
 };
 
 // ---------------------------------------------------------------------------------------
-// FP64 stage kernel, Y form. Each thread owns VEC consecutive columns and marches down RY
-// rows keeping rows j-1, j, j+1 of Y_{j-1} in registers; W/E neighbours at the thread's
-// edge come through L1. One read of each input stream, one write of Y_j.
+// FP64 stage kernel, Y form. Each thread owns one column and marches down RY rows keeping rows
+// j-1, j, j+1 of Y_{j-1} in registers; W/E neighbours come through L1. One read of each input
+// stream, one write of Y_j.
+// Large grids are bound by the FP64 pipe (10 instructions per forced point at 1.6 lanes per
+// clock and SM): the two neighbour sums, the product with gc and the F_0 term (|gf F_0| well
+// below the accumulator away from its zeros) run as integer code (soft64.cuh), which leaves 6
+// FP64 instructions beside them. 4096^2, forced: 312 us per stage with all ten in FP64, 219 us
+// so; with the sums only 268, sums and product 253, with g0 Y_0 as integer code too 245 (then
+// the integer side bounds it), the small term without the product 231. Two columns per thread
+// are no faster (62.6 against 62.0 us at 2048^2) and slower on small grids; with 8 rows five
+// blocks per SM (219 us at 4096^2; four 227, six 222, three 251), else four.
+// Small grids are bound by the latency of the rows that one thread takes in turn (about 1 us
+// each): see launch_stage64 for the rows per thread.
 // ---------------------------------------------------------------------------------------
-template <int VEC, int RY, bool FORCED>
-__global__ void __launch_bounds__(256) stage64_kernel(ProbDev P, const StageArgs* __restrict__ A,
-                                                      const double* __restrict__ ym1,
-                                                      const double* __restrict__ ym2,
-                                                      const double* __restrict__ y0,
-                                                      const double* __restrict__ f0,
-                                                      double* __restrict__ yj)
+template <int RY, bool FORCED>
+__global__ void __launch_bounds__(256, RY == 8 ? 5 : 4) stage64_kernel(ProbDev P, const StageArgs* __restrict__ A,
+                                                         const double* __restrict__ ym1,
+                                                         const double* __restrict__ ym2,
+                                                         const double* __restrict__ y0,
+                                                         const double* __restrict__ f0,
+                                                         double* __restrict__ yj)
 {
-  using IO           = VecIO<double, VEC>;
   const long long nx = P.nx, ny = P.ny;
-  const long long i0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * VEC;
+  const long long i  = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long jb = ((long long)blockIdx.y * blockDim.y + threadIdx.y) * RY;
-  if (i0 >= nx || jb >= ny) return;
+  if (i >= nx || jb >= ny) return;
   const long long je = (jb + RY < ny) ? jb + RY : ny;
-  // the thread's VEC-wide loads and stores stay inside the row
-  if (!STS_IN_BOUNDS(i0 + VEC <= nx && i0 % VEC == 0, P.err)) return;
+  if (!STS_IN_BOUNDS(jb * nx + i < nx * ny && (je - 1) * nx + i < nx * ny, P.err)) return;
   const double gc = A->gc, gx = A->gx, gy = A->gy, gn = A->gn, g0 = A->g0, gf = A->gf;
-  double Pi[VEC], Qi[VEC];
+  const soft64::Factor gcF = soft64::factor(gc), gfF = soft64::factor(gf);
+  double Pi = 0.0, Qi = 0.0;
   if (FORCED)
   {
-    const double al = A->al, be = A->be, ga = A->ga;
-#pragma unroll
-    for (int v = 0; v < VEC; ++v)
-    {
-      Pi[v] = __fma_rn(al, P.Sx[i0 + v], be * P.Sxx[i0 + v]);
-      Qi[v] = ga * P.Sx[i0 + v];
-    }
+    Pi = __fma_rn(A->al, P.Sx[i], A->be * P.Sxx[i]);
+    Qi = A->ga * P.Sx[i];
   }
-  double up[VEC], cur[VEC], dn[VEC];
-  if (jb > 0) IO::ld(ym1 + (jb - 1) * nx + i0, up);
-  else
-#pragma unroll
-    for (int v = 0; v < VEC; ++v) up[v] = 0.0;
-  IO::ld(ym1 + jb * nx + i0, cur);
+  double up  = jb > 0 ? __ldg(ym1 + (jb - 1) * nx + i) : 0.0;
+  double cur = __ldg(ym1 + jb * nx + i);
+#pragma unroll 1
   for (long long j = jb; j < je; ++j)
   {
-    const long long row = j * nx + i0;
-    if (j + 1 < ny) IO::ld(ym1 + row + nx, dn);
-    else
-#pragma unroll
-      for (int v = 0; v < VEC; ++v) dn[v] = 0.0;
-    const double w = (i0 > 0) ? __ldg(ym1 + row - 1) : 0.0;
-    const double e = (i0 + VEC < nx) ? __ldg(ym1 + row + VEC) : 0.0;
-    double m2[VEC], z0[VEC], q0[VEC], out[VEC];
-    IO::ld(ym2 + row, m2);
-    IO::ld(y0 + row, z0);
-    IO::ld(f0 + row, q0);
-    double syj = 0.0, syyj = 0.0;
+    const long long k = j * nx + i;
+    const double dn = (j + 1 < ny) ? __ldg(ym1 + k + nx) : 0.0;
+    const double w  = (i > 0) ? __ldg(ym1 + k - 1) : 0.0;
+    const double e  = (i + 1 < nx) ? __ldg(ym1 + k + 1) : 0.0;
+    const double m2 = __ldg(ym2 + k), z0 = __ldg(y0 + k), q0 = __ldg(f0 + k);
+    const double sx = s64_add(w, e), sy = s64_add(up, dn);
+    double acc      = s64_mul(gcF, gc, cur);
+    acc             = __fma_rn(gx, sx, acc);
+    acc             = __fma_rn(gy, sy, acc);
+    acc             = __fma_rn(gn, m2, acc);
+    acc             = __fma_rn(g0, z0, acc);
+    acc             = s64_fma_small(gfF, gf, q0, acc);
     if (FORCED)
     {
-      syj  = __ldg(P.Sy + j);
-      syyj = __ldg(P.Syy + j);
+      acc = __fma_rn(__ldg(P.Sy + j), Pi, acc);
+      acc = __fma_rn(__ldg(P.Syy + j), Qi, acc);
     }
-#pragma unroll
-    for (int v = 0; v < VEC; ++v)
-    {
-      const double uw = (v == 0) ? w : cur[v - 1];
-      const double ue = (v == VEC - 1) ? e : cur[v + 1];
-      const double sx = uw + ue, sy = up[v] + dn[v];
-      double acc      = gc * cur[v];
-      acc             = __fma_rn(gx, sx, acc);
-      acc             = __fma_rn(gy, sy, acc);
-      acc             = __fma_rn(gn, m2[v], acc);
-      acc             = __fma_rn(g0, z0[v], acc);
-      acc             = __fma_rn(gf, q0[v], acc);
-      if (FORCED)
-      {
-        acc = __fma_rn(syj, Pi[v], acc);
-        acc = __fma_rn(syyj, Qi[v], acc);
-      }
-      out[v] = acc;
-    }
-    IO::st(yj + row, out);
-#pragma unroll
-    for (int v = 0; v < VEC; ++v)
-    {
-      up[v]  = cur[v];
-      cur[v] = dn[v];
-    }
+    yj[k] = acc;
+    up    = cur;
+    cur   = dn;
   }
 }
 

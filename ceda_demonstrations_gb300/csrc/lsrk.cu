@@ -566,9 +566,8 @@ static int ensure_par(LSRKMem* m)
 // ---------------------------------------------------------------------------------------
 // fused stage loop
 // ---------------------------------------------------------------------------------------
-// launch shapes: FP64 stage 64x4 threads, 2 columns x 8 rows per thread; FP32 stage 64x4
-// threads, 4 columns x 8 rows per thread; scalar-column variants when nx is not a
-// multiple of the vector width.
+// launch shapes: FP64 stage 64x4 threads (launch_stage64); FP32 stage 64x4 threads, 4 columns x
+// 8 rows per thread; scalar-column variants when nx is not a multiple of the vector width.
 static constexpr int RY = 8;
 
 template <typename F>
@@ -578,25 +577,29 @@ static void dispatch_forced(bool forced, F&& f)
   else f(std::false_type{});
 }
 
+// Rows per thread of the FP64 stage: fewer neighbour loads with more rows, but a thread takes
+// its rows one after another. One row until the points fill the resident threads once (W: four
+// blocks of 256 per SM), then 2, 4 and 8 rows as the grid gets waves to spare. Measured us per
+// stage with 1 / 2 / 4 / 8 rows: 128^2 3.3 / 4.1 / 5.8 / 9.0, 384^2 5.16 / 5.12 / 6.1 / 9.8,
+// 512^2 7.2 / 7.2 / 7.4 / 9.5, 1024^2 20.3 / 18.2 / 17.7 / 19.3, 2048^2 82 / 70 / 63.5 / 62.0.
 static void launch_stage64(LSRKMem* m, STS_Problem p, const StageArgs* A, const double* ym1, const double* ym2,
                            const double* y0, const double* f0, double* yj)
 {
   const bool forced = p->kind == STS_PROBLEM_MANUFACTURED;
   dim3 b(64, 4);
-  if (p->nx % 2 == 0)
-  {
-    dim3 g((unsigned)((p->nx / 2 + b.x - 1) / b.x), (unsigned)((p->ny + b.y * RY - 1) / (b.y * RY)));
+  auto go = [&](auto Rc) {
+    constexpr int R = decltype(Rc)::value;
+    dim3 g((unsigned)((p->nx + b.x - 1) / b.x), (unsigned)((p->ny + b.y * R - 1) / (b.y * R)));
     dispatch_forced(forced, [&](auto F) {
-      stage64_kernel<2, RY, decltype(F)::value><<<g, b, 0, m->ctx->stream>>>(p->dev, A, ym1, ym2, y0, f0, yj);
+      stage64_kernel<R, decltype(F)::value><<<g, b, 0, m->ctx->stream>>>(p->dev, A, ym1, ym2, y0, f0, yj);
     });
-  }
-  else
-  {
-    dim3 g((unsigned)((p->nx + b.x - 1) / b.x), (unsigned)((p->ny + b.y * RY - 1) / (b.y * RY)));
-    dispatch_forced(forced, [&](auto F) {
-      stage64_kernel<1, RY, decltype(F)::value><<<g, b, 0, m->ctx->stream>>>(p->dev, A, ym1, ym2, y0, f0, yj);
-    });
-  }
+  };
+  const long long n = p->nx * p->ny, W = 1024LL * m->ctx->num_sms;
+  const long long nyb = p->ny / (4 * 65535); // the grid's second dimension ends at 65535 blocks
+  if (n < W && nyb < 1) go(std::integral_constant<int, 1>{});
+  else if (n < 3 * W && nyb < 2) go(std::integral_constant<int, 2>{});
+  else if (n < 10 * W && nyb < 4) go(std::integral_constant<int, 4>{});
+  else go(std::integral_constant<int, 8>{});
 }
 
 static void launch_stage32(LSRKMem* m, STS_Problem p, const StageArgs* A, const float* dm1, const float* dm2,

@@ -508,3 +508,26 @@ def test_evolve_rejects_bad_arguments(ctx, stslib):
     J = stslib.LSRKStep(ctx, G, 0.0, G.initial(), method=1, hfixed=1.0, smax=10)
     assert L.STS_ARKodeEvolve(J.mem, 0.5, y.h, C.byref(t), stslib.NORMAL) == STS_ILL_INPUT
 
+
+
+@pytest.mark.parametrize("nx,ny", [(390, 398), (391, 401), (683, 683), (1247, 1250), (1248, 1249)])
+@pytest.mark.parametrize("kind", [0, 1])
+def test_fp64_stage_rows_per_thread_bitwise(ctx, stslib, oracle, nx, ny, kind):
+    """The FP64 stage on both sides of the sizes where its rows per thread change (1, 2, 4 and 8
+    rows: 1, 3 and 10 times 1024 points per SM), with ragged last rows, forced and unforced: one
+    fixed step, bit for bit."""
+    P = stslib.Problem(ctx, kind, nx, ny, 1.0, 0.3)
+    O = oracle.Problem(kind, nx, ny, 1.0, 0.3)
+    if kind:
+        modes = (np.array([1, 5]), np.array([2, 3]), np.array([1.0, -0.4]))
+        y0, yo = P.initial_modes(*modes), O.initial_modes(*modes)
+    else:
+        y0, yo = P.initial(), O.initial()
+    h = 30.0 / (8.0 * max(nx * nx, ny * ny))
+    I = stslib.LSRKStep(ctx, P, 0.0, y0, method=1, rtol=1e-6, atol=1e-10, hfixed=h)
+    J = oracle.Integrator(O, yo, method=1, rtol=1e-6, atol=1e-10, hfixed=h)
+    y = P.vector()
+    I.evolve(h, y)
+    assert J.evolve(h) == 0
+    assert I.stats()["nst"] == 1 and I.stats()["stage_max"] >= 5
+    assert np.array_equal(y.numpy(), J.y)
