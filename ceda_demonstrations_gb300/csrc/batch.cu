@@ -172,24 +172,9 @@ template <int NT, int CL>
 __device__ double inst_exact_sum(xsum::Limbs& a, unsigned flags, long long (*sm)[xsum::NL], long long* climb,
                                  unsigned* cflags, double* sres)
 {
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (tid == 0) *cflags = 0;
-#pragma unroll
-  for (int k = 0; k < xsum::NL; ++k)
-  {
-    long long v = a.l[k];
-#pragma unroll
-    for (int m = 16; m >= 1; m >>= 1) v += shfl_xor_ll(v, m);
-    if (lane == 0) sm[warp][k] = v;
-  }
-  __syncthreads();
-  if (flags) atomicOr(cflags, flags);
-  if (tid < xsum::NL)
-  {
-    long long v = 0;
-    for (int w = 0; w < NT / 32; ++w) v += sm[w][tid];
-    climb[tid] = v;
-  }
+  const int tid     = threadIdx.x;
+  const long long v = xsum_block_limbs<NT>(a, &flags, sm, cflags);
+  if (tid < xsum::NL) climb[tid] = v;
   inst_sync<CL>(); // climb[] and cflags of every CTA complete
   if (tid == 0)
   {

@@ -113,65 +113,77 @@ __device__ __forceinline__ long long shfl_xor_ll(long long v, int m)
   return (long long)__shfl_xor_sync(0xffffffffu, (unsigned long long)v, m);
 }
 
+// 64-bit sum over the lanes of a full warp, on the integer reduction instruction: 24-bit
+// digits (32 of them fit 29 bits), the highest one signed.
+__device__ __forceinline__ long long warp_sum_ll(long long v)
+{
+  const unsigned lo = __reduce_add_sync(0xffffffffu, (unsigned)v & 0xffffffu);
+  const unsigned mi = __reduce_add_sync(0xffffffffu, (unsigned)(v >> 24) & 0xffffffu);
+  const int hi      = __reduce_add_sync(0xffffffffu, (int)(v >> 48));
+  return (long long)lo + ((long long)mi << 24) + (long long)((unsigned long long)(long long)hi << 48);
+}
+
+// Exact sums of a block: every thread passes its limbs; lane k < NL of warp 0 returns limb k
+// of the block's total, and every thread the union of the flags. The terms of a block usually
+// span a few limbs, so limbs that are zero in the whole warp cost one vote. `sm` is shared.
+template <int NT>
+__device__ __forceinline__ long long xsum_block_limbs(const xsum::Limbs& a, unsigned* flags,
+                                                      long long (*sm)[xsum::NL], unsigned* sflags)
+{
+  // linear thread index: blocks may be 1-D or 2-D (NT threads in total)
+  const int tid  = threadIdx.x + blockDim.x * (threadIdx.y + blockDim.y * threadIdx.z);
+  const int lane = tid & 31, warp = tid >> 5;
+  if (tid == 0) *sflags = 0;
+#pragma unroll
+  for (int k = 0; k < xsum::NL; ++k)
+  {
+    long long v = 0;
+    if (__any_sync(0xffffffffu, a.l[k] != 0)) v = warp_sum_ll(a.l[k]);
+    if (lane == 0) sm[warp][k] = v;
+  }
+  if (__syncthreads_or(*flags))
+  { // NaN or overflow: the union of the bits
+    if (*flags) atomicOr(sflags, *flags);
+    __syncthreads();
+    *flags = *sflags;
+  }
+  long long v = 0;
+  if (tid < xsum::NL)
+#pragma unroll
+    for (int w = 0; w < NT / 32; ++w) v += sm[w][tid];
+  return v;
+}
+
 // Block-level combine of per-thread limbs, then global atomics + last-block finalisation.
 // Every thread of the block must call it. `post` selects the final transform:
 //   0: value, 1: sqrt(value / n) (WRMS). The result goes to slot_out.
+// Small reductions are all latency: one barrier, the limbs of a block added, fetched and
+// cleared by one lane each, and a register-only finalisation.
 template <int NT>
 __device__ __forceinline__ void xsum_block_finish(xsum::Limbs& a, unsigned flags, RedWork* w,
                                                   double* slot_out, int post, double n)
 {
   __shared__ long long sm[NT / 32][xsum::NL];
   __shared__ unsigned sflags;
-  __shared__ bool last;
-  // linear thread index: blocks may be 1-D or 2-D (NT threads in total)
-  const int tid  = threadIdx.x + blockDim.x * (threadIdx.y + blockDim.y * threadIdx.z);
-  const int lane = tid & 31, warp = tid >> 5;
-  if (tid == 0) sflags = 0;
-#pragma unroll
-  for (int k = 0; k < xsum::NL; ++k)
-  {
-    long long v = a.l[k];
-#pragma unroll
-    for (int m = 16; m >= 1; m >>= 1) v += shfl_xor_ll(v, m);
-    if (lane == 0) sm[warp][k] = v;
-  }
-  __syncthreads();
-  if (flags) atomicOr(&sflags, flags);
-  if (warp == 0)
-  {
-#pragma unroll
-    for (int k = 0; k < xsum::NL; ++k)
-    {
-      long long v = (lane < NT / 32) ? sm[lane][k] : 0LL;
-#pragma unroll
-      for (int m = 16; m >= 1; m >>= 1) v += shfl_xor_ll(v, m);
-      if (lane == 0 && v != 0) atomicAdd(&w->limbs[k], (unsigned long long)v);
-    }
-  }
-  __syncthreads();
+  const int tid = threadIdx.x + blockDim.x * (threadIdx.y + blockDim.y * threadIdx.z);
+  const long long v = xsum_block_limbs<NT>(a, &flags, sm, &sflags);
+  if (tid >= 32) return;
+  if (tid < xsum::NL && v != 0) atomicAdd(&w->limbs[tid], (unsigned long long)v);
+  if (tid == 0 && flags) atomicOr(&w->flags, flags);
+  __threadfence();
+  __syncwarp();
+  unsigned t = 0;
+  if (tid == 0) t = atomicAdd(&w->ticket, 1u);
+  t = __shfl_sync(0xffffffffu, t, 0);
+  if (t != gridDim.x * gridDim.y * gridDim.z - 1) return;
+  __threadfence();
+  if (tid < xsum::NL) sm[0][tid] = (long long)atomicExch(&w->limbs[tid], 0ULL);
+  __syncwarp();
   if (tid == 0)
   {
-    if (sflags) atomicOr(&w->flags, sflags);
-    __threadfence();
-    unsigned t = atomicAdd(&w->ticket, 1u);
-    last       = (t == gridDim.x * gridDim.y * gridDim.z - 1);
-  }
-  __syncthreads();
-  if (last && tid == 0)
-  {
-    __threadfence();
-    long long tot[xsum::NL];
-#pragma unroll
-    for (int k = 0; k < xsum::NL; ++k)
-    {
-      tot[k]       = (long long)atomicAdd(&w->limbs[k], 0ULL);
-      w->limbs[k]  = 0ULL;
-    }
-    unsigned f = atomicOr(&w->flags, 0u);
-    double v   = xsum::finalize(tot, f);
-    if (post == 1) v = sqrt(v / n);
-    *slot_out = v;
-    w->flags  = 0u;
+    double r = xsum::finalize(sm[0], atomicExch(&w->flags, 0u));
+    if (post == 1) r = sqrt(r / n);
+    *slot_out = r;
     w->ticket = 0u;
     __threadfence();
   }

@@ -15,6 +15,8 @@
 #include <cstdint>
 #include <cstring>
 
+#include "soft64.cuh"
+
 #ifdef __CUDACC__
 #define XS_HD __host__ __device__ __forceinline__
 #else
@@ -132,7 +134,8 @@ XS_HD double from_bits(unsigned long long b)
 
 // Normalise the limbs into a two's-complement integer of 32-bit digits and round it to the
 // nearest double (ties to even). Integer arithmetic only, so host and device produce the
-// same bits.
+// same bits; no array is indexed by a computed value, so the device keeps it in registers (one
+// thread runs this at the end of every reduction).
 XS_HD double finalize(const long long* limbs, unsigned flags)
 {
   if (flags & FLAG_NAN) return from_bits(0x7ff8000000000000ULL);
@@ -140,78 +143,48 @@ XS_HD double finalize(const long long* limbs, unsigned flags)
   constexpr int ND = NL + 1; // digit NL holds the sign extension
   unsigned int dg[ND];
   long long carry = 0;
+#pragma unroll
   for (int k = 0; k < NL; ++k)
   {
-    long long v = limbs[k] + carry;
-    dg[k]       = (unsigned int)(v & 0xffffffffLL);
-    carry       = v >> 32; // arithmetic shift: floor division by 2^32
+    const long long v = limbs[k] + carry;
+    dg[k]             = (unsigned int)(v & 0xffffffffLL);
+    carry             = v >> 32; // arithmetic shift: floor division by 2^32
   }
   const bool negative = carry < 0;
   dg[NL]              = (unsigned int)(carry & 0xffffffffLL);
   if (negative)
   { // magnitude = two's-complement negation
     unsigned long long c = 1;
+#pragma unroll
     for (int k = 0; k < ND; ++k)
     {
-      unsigned long long s = (unsigned long long)(unsigned int)(~dg[k]) + c;
-      dg[k]                = (unsigned int)s;
-      c                    = s >> 32;
+      const unsigned long long s = (unsigned long long)(unsigned int)(~dg[k]) + c;
+      dg[k]                      = (unsigned int)s;
+      c                          = s >> 32;
     }
   }
+  // the three highest digits from the leading nonzero one, and whether anything lies below
   int top = -1;
-  for (int k = ND - 1; k >= 0 && top < 0; --k)
-    if (dg[k])
+  unsigned int w2 = 0, w1 = 0, w0 = 0, below = 0;
+#pragma unroll
+  for (int k = ND - 1; k >= 0; --k)
+  {
+    if (top < 0)
     {
-      int msb = 31;
-      while (!((dg[k] >> msb) & 1u)) --msb;
-      top = k * 32 + msb;
+      w2  = dg[k];
+      top = w2 ? k : -1;
     }
+    else if (top - k == 1) w1 = dg[k];
+    else if (top - k == 2) w0 = dg[k];
+    else below |= dg[k];
+  }
   if (top < 0) return 0.0;
-  int shift = top - 52;
-  unsigned long long mant;
-  if (shift <= 0)
-  { // the magnitude fits in 53 bits: exact
-    mant  = (unsigned long long)dg[0] | ((unsigned long long)dg[1] << 32);
-    shift = 0;
-  }
-  else
-  {
-    const int k = shift >> 5, b = shift & 31;
-    unsigned long long w0 = dg[k];
-    unsigned long long w1 = (k + 1 < ND) ? dg[k + 1] : 0ULL;
-    unsigned long long w2 = (k + 2 < ND) ? dg[k + 2] : 0ULL;
-    unsigned long long c  = w0 | (w1 << 32);
-    mant                  = (c >> b) | (b ? (w2 << (64 - b)) : 0ULL);
-    mant &= ((1ULL << 53) - 1);
-    const int r  = shift - 1;
-    const bool rb = ((dg[r >> 5] >> (r & 31)) & 1u) != 0;
-    bool sticky   = (dg[r >> 5] & ((1u << (r & 31)) - 1u)) != 0;
-    for (int q = 0; q < (r >> 5); ++q) sticky = sticky || (dg[q] != 0);
-    if (rb && (sticky || (mant & 1ULL)))
-    {
-      mant++;
-      if (mant == (1ULL << 53))
-      {
-        mant >>= 1;
-        shift++;
-      }
-    }
-  }
-  // value = mant * 2^(shift - 160): exact power-of-two scaling in steps of 2^60
-  double v = (double)mant;
-  int ex   = shift - 160;
-  while (ex <= -60)
-  {
-    v *= 0x1p-60;
-    ex += 60;
-  }
-  while (ex >= 60)
-  {
-    v *= 0x1p60;
-    ex -= 60;
-  }
-  v *= (ex < 0) ? 1.0 / (double)(1ULL << (-ex)) : (double)(1ULL << ex);
-  return negative ? -v : v;
+  // leading one to bit 63, the rest as a sticky bit
+  const int lz               = soft64::leading_zeros(w2);
+  const unsigned long long m = ((((unsigned long long)w2 << 32) | w1) << lz) | (((unsigned long long)w0 << lz) >> 32);
+  below |= w0 << lz;
+  const int e = 1023 - 160 + 32 * top + 31 - lz; // exponent field of the leading one
+  return soft64::round_pack(negative ? 0x80000000u : 0u, e, m | (below ? 1u : 0u));
 }
 
 } // namespace xsum
