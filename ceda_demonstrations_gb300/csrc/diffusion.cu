@@ -113,6 +113,7 @@ extern "C" STS_Problem STS_ProblemCreate(STS_Context ctx, int kind, sts_index nx
   d.err      = ctx->d_err;
   d.nx       = nx;
   d.ny       = ny;
+  d.ldf      = (nx + 3) / 4 * 4;
   d.kind     = kind;
   d.inhom    = p->inhom;
   d.kx       = kx;

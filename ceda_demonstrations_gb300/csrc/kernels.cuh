@@ -110,34 +110,6 @@ __device__ __forceinline__ float mixed_point(float gs, float gx, float gy, float
   return __fadd_rn(dc, inc);
 }
 
-// mixed_point on two points at once with the paired FP32 instructions of sm_100 and later
-// (__fadd2_rn, __fmul2_rn, __ffma2_rn: per component the same rounding as __fadd_rn,
-// __fmul_rn, __fmaf_rn). A difference a - b is taken as a + (-b), which IEEE arithmetic gives
-// exactly, signed zeros included; the negations are multiplications by -1 (exact). The two
-// components are bit-identical to two mixed_point calls. Operands are (point 0, point 1)
-// pairs; the scalars arrive duplicated.
-template <bool FORCED>
-__device__ __forceinline__ float2 mixed_pair(float2 gs, float2 gx, float2 gy, float2 gm, float2 gF, float2 dc,
-                                             float2 dw, float2 de, float2 ds, float2 dn, float2 m2, float2 q0,
-                                             float2 syj, float2 pi, float2 syyj, float2 qi)
-{
-  const float2 neg1 = make_float2(-1.0f, -1.0f);
-  const float2 ndc  = __fmul2_rn(dc, neg1);
-  const float2 lx   = __fadd2_rn(__fadd2_rn(dw, ndc), __fadd2_rn(de, ndc));
-  const float2 ly   = __fadd2_rn(__fadd2_rn(ds, ndc), __fadd2_rn(dn, ndc));
-  float2 inc        = __fmul2_rn(gs, dc);
-  inc               = __ffma2_rn(gx, lx, inc);
-  inc               = __ffma2_rn(gy, ly, inc);
-  inc               = __ffma2_rn(gm, __fadd2_rn(dc, __fmul2_rn(m2, neg1)), inc);
-  inc               = __ffma2_rn(gF, q0, inc);
-  if (FORCED)
-  {
-    inc = __ffma2_rn(syj, pi, inc);
-    inc = __ffma2_rn(syyj, qi, inc);
-  }
-  return __fadd2_rn(dc, inc);
-}
-
 // Error weight of the mixed form's step end, 1 / (rtol |y| + atol) to within a few ulp with five
 // FP64-pipe operations instead of a correctly rounded division (about ten on GB300, whose FP64
 // pipe bounds this kernel): den = fma(rtol, |y|, atol), the correctly rounded FP32 reciprocal of
@@ -278,7 +250,7 @@ __global__ void __launch_bounds__(256) stage32_kernel(ProbDev P, const StageArgs
                                                       float* __restrict__ dj)
 {
   using IO           = VecIO<float, VEC>;
-  const long long nx = P.nx, ny = P.ny;
+  const long long nx = P.nx, ny = P.ny, ld = P.ldf;
   const long long i0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * VEC;
   const long long jb = ((long long)blockIdx.y * blockDim.y + threadIdx.y) * RY;
   if (i0 >= nx || jb >= ny) return;
@@ -299,15 +271,15 @@ __global__ void __launch_bounds__(256) stage32_kernel(ProbDev P, const StageArgs
     }
   }
   float up[VEC], cur[VEC], dn[VEC];
-  if (jb > 0) IO::ld(dm1 + (jb - 1) * nx + i0, up);
+  if (jb > 0) IO::ld(dm1 + (jb - 1) * ld + i0, up);
   else
 #pragma unroll
     for (int v = 0; v < VEC; ++v) up[v] = 0.0f;
-  IO::ld(dm1 + jb * nx + i0, cur);
+  IO::ld(dm1 + jb * ld + i0, cur);
   for (long long j = jb; j < je; ++j)
   {
-    const long long row = j * nx + i0;
-    if (j + 1 < ny) IO::ld(dm1 + row + nx, dn);
+    const long long row = j * ld + i0;
+    if (j + 1 < ny) IO::ld(dm1 + row + ld, dn);
     else
 #pragma unroll
       for (int v = 0; v < VEC; ++v) dn[v] = 0.0f;
@@ -401,15 +373,15 @@ __global__ void __launch_bounds__(256) stepend_kernel(ProbDev P, const StepArgs*
     }
     for (long long j = blockIdx.y; j < ny; j += gridDim.y)
     {
-      const long long k = j * nx + i;
+      const long long k = j * nx + i, kf = j * P.ldf + i;
       double uc, uw, ue, us, un;
       if (MIXED)
       {
-        uc = yn[k] + (double)ds[k];
-        uw = (i > 0) ? yn[k - 1] + (double)ds[k - 1] : 0.0;
-        ue = (i < nx - 1) ? yn[k + 1] + (double)ds[k + 1] : 0.0;
-        us = (j > 0) ? yn[k - nx] + (double)ds[k - nx] : 0.0;
-        un = (j < ny - 1) ? yn[k + nx] + (double)ds[k + nx] : 0.0;
+        uc = yn[k] + (double)ds[kf];
+        uw = (i > 0) ? yn[k - 1] + (double)ds[kf - 1] : 0.0;
+        ue = (i < nx - 1) ? yn[k + 1] + (double)ds[kf + 1] : 0.0;
+        us = (j > 0) ? yn[k - nx] + (double)ds[kf - P.ldf] : 0.0;
+        un = (j < ny - 1) ? yn[k + nx] + (double)ds[kf + P.ldf] : 0.0;
       }
       else
       {
@@ -432,11 +404,11 @@ __global__ void __launch_bounds__(256) stepend_kernel(ProbDev P, const StepArgs*
       if (MIXED)
       {
         ynew[k]  = uc;
-        Fnewf[k] = (float)f;
+        Fnewf[kf] = (float)f;
       }
       const double y = yn[k];
       // the mixed form takes y_n - y_{n+1} as -d_s itself (exact) and the fast weight
-      const double d = MIXED ? -(double)ds[k] : y - uc;
+      const double d = MIXED ? -(double)ds[kf] : y - uc;
       double e       = 0.8 * d;
       e              = __fma_rn(p4h, Fn[k], e);
       e              = __fma_rn(p4h, f, e);
@@ -486,7 +458,7 @@ __global__ void __launch_bounds__(256) stepend_march_kernel(ProbDev P, const Ste
     if (MIXED)
     {
       const double2 a = __ldg(reinterpret_cast<const double2*>(yn + k));
-      const float2 b  = __ldg(reinterpret_cast<const float2*>(ds + k));
+      const float2 b  = __ldg(reinterpret_cast<const float2*>(ds + j * P.ldf + i0));
       v[0]            = a.x + (double)b.x;
       v[1]            = a.y + (double)b.y;
     }
@@ -500,7 +472,7 @@ __global__ void __launch_bounds__(256) stepend_march_kernel(ProbDev P, const Ste
   auto point = [&](long long j, long long i) -> double { // single y_{n+1} value (edges)
     if (i < 0 || i >= nx || j < 0 || j >= ny) return 0.0;
     const long long k = j * nx + i;
-    return MIXED ? yn[k] + (double)ds[k] : Ys[k];
+    return MIXED ? yn[k] + (double)ds[j * P.ldf + i] : Ys[k];
   };
   double Pi[2] = {0.0, 0.0}, Qi[2] = {0.0, 0.0};
   if (FORCED && colok)
@@ -536,7 +508,7 @@ __global__ void __launch_bounds__(256) stepend_march_kernel(ProbDev P, const Ste
       float dsv[2] = {0.f, 0.f};
       if (MIXED)
       {
-        const float2 t = __ldg(reinterpret_cast<const float2*>(ds + k));
+        const float2 t = __ldg(reinterpret_cast<const float2*>(ds + j * P.ldf + i0));
         dsv[0]         = t.x;
         dsv[1]         = t.y;
       }
@@ -575,7 +547,7 @@ __global__ void __launch_bounds__(256) stepend_march_kernel(ProbDev P, const Ste
       if (MIXED)
       {
         *reinterpret_cast<double2*>(ynew + k) = make_double2(cur[0], cur[1]);
-        *reinterpret_cast<float2*>(Fnewf + k) = make_float2((float)fo[0], (float)fo[1]);
+        *reinterpret_cast<float2*>(Fnewf + j * P.ldf + i0) = make_float2((float)fo[0], (float)fo[1]);
       }
     }
 #pragma unroll

@@ -33,6 +33,7 @@
 #include "sts_internal.cuh"
 
 void sts_f64_to_f32(STS_Context ctx, const double* a, float* b, long long n);
+static void field_to_f32(STS_Context ctx, STS_Problem p, const double* a, float* b);
 
 // ---------------------------------------------------------------------------------------
 // coefficient and step-size rules (host)
@@ -244,6 +245,11 @@ struct LSRKMem {
   int fuse_req = 0, fuse_tile_req = -1;
   int fuse_ks = 1, fuse_ti = -1;
   double fuse_ms[TMA_FUSED_NTILES] = {};
+  // groups of 8 stages: the autotuner's tile configuration (-1: none) and its time per launch;
+  // the rest of a step runs in groups of fuse_ks
+  int deep_ti    = -1;
+  double deep_ms = 0.0;
+  long long f32_nx = 0, f32_ny = 0; // the grid that the FP32 buffers and their tensor maps fit
   long long n           = 0;
 
   // state (mirrors the oracle's orc_state)
@@ -503,30 +509,70 @@ static StageArgs* hstage(LSRKMem* m) { return (StageArgs*)((char*)m->h_par + siz
 static StepArgs* dstep(LSRKMem* m) { return (StepArgs*)m->d_par; }
 static StageArgs* dstage(LSRKMem* m) { return (StageArgs*)((char*)m->d_par + sizeof(StepArgs) + 8); }
 
+// bytes of an FP32 field of the fused path (rows padded to ProbDev::ldf)
+static size_t f32_field_bytes(const LSRKMem* m)
+{
+  const STS_Problem p = (STS_Problem)m->user_data;
+  return (size_t)(p->dev.ldf * p->ny) * sizeof(float);
+}
+
 // allocate the fused-path buffers (y0 copied into yb[0])
 static int alloc_fused(LSRKMem* m, const double* y0dev)
 {
-  const size_t n8 = m->n * sizeof(double), n4 = m->n * sizeof(float);
+  const size_t n8 = m->n * sizeof(double), n4 = f32_field_bytes(m);
   cudaStream_t st = m->ctx->stream;
   for (int b = 0; b < 2; ++b)
   {
     if (!STS_CUDA_OK(cudaMalloc(&m->yb[b], n8)) || !STS_CUDA_OK(cudaMalloc(&m->Fb[b], n8)) ||
-        !STS_CUDA_OK(cudaMalloc(&m->Ffb[b], n4)))
+        !STS_CUDA_OK(cudaMalloc(&m->Ffb[b], n4)) || !STS_CUDA_OK(cudaMemsetAsync(m->Ffb[b], 0, n4, st)))
       return -1;
   }
   m->par_bytes = sizeof(StepArgs) + 8 + sizeof(StageArgs) * (size_t)(m->smax + 1);
   if (!STS_CUDA_OK(cudaMalloc(&m->d_par, m->par_bytes)) ||
       !STS_CUDA_OK(cudaHostAlloc(&m->h_par, m->par_bytes, cudaHostAllocDefault)))
     return -1;
+  m->f32_nx = ((STS_Problem)m->user_data)->nx;
+  m->f32_ny = ((STS_Problem)m->user_data)->ny;
   memset(m->h_par, 0, m->par_bytes);
   if (!STS_CUDA_OK(cudaMemcpyAsync(m->yb[0], y0dev, n8, cudaMemcpyDeviceToDevice, st))) return -1;
   m->par = 0;
   return 0;
 }
 
+// after ARKodeSetUserData with a problem of another grid shape (the same number of points): FP32
+// buffers of that shape's pitch, with the FP32 copy of F_n
+static int refit_f32(LSRKMem* m)
+{
+  STS_Problem p = (STS_Problem)m->user_data;
+  if (m->f32_nx == p->nx && m->f32_ny == p->ny) return 0;
+  if (!STS_CUDA_OK(cudaStreamSynchronize(m->ctx->stream))) return -1;
+  for (auto& kv : m->graphs) cudaGraphExecDestroy(kv.second);
+  m->graphs.clear();
+  for (int b = 0; b < 4; ++b)
+  {
+    cudaFree(m->D[b]);
+    m->D[b] = nullptr;
+  }
+  const size_t n4 = f32_field_bytes(m);
+  for (int b = 0; b < 2; ++b)
+  {
+    cudaFree(m->Ffb[b]);
+    m->Ffb[b] = nullptr;
+    if (!STS_CUDA_OK(cudaMalloc(&m->Ffb[b], n4)) || !STS_CUDA_OK(cudaMemsetAsync(m->Ffb[b], 0, n4, m->ctx->stream)))
+      return -1;
+  }
+  if (m->mixed && m->initialized) field_to_f32(m->ctx, p, m->Fb[m->par], m->Ffb[m->par]);
+  m->tma.ok = m->tma.fz_ok = false;
+  m->tuned  = false;
+  m->f32_nx = p->nx;
+  m->f32_ny = p->ny;
+  return 0;
+}
+
 static int ensure_stage_buffers(LSRKMem* m)
 {
-  const size_t n8 = m->n * sizeof(double), n4 = m->n * sizeof(float);
+  if (refit_f32(m)) return -1;
+  const size_t n8 = m->n * sizeof(double), n4 = f32_field_bytes(m);
   for (int b = 0; b < 3; ++b)
   {
     if (!m->mixed && !m->Y[b] && !STS_CUDA_OK(cudaMalloc(&m->Y[b], n8))) return -1;
@@ -622,16 +668,33 @@ static void launch_stage32_idx(LSRKMem* m, STS_Problem p, const StageArgs* A, in
   launch_stage32_idx(m, p, A, im1, im2, par, iout, v);
 }
 
-// Autotuner for the mixed stage kernel: times every TMA configuration and the register
-// kernel on the integrator's own buffers (a realistic stage, CUDA events on the context
-// stream, 2 warm + 5 timed launches each) and keeps the fastest for this problem.
+// Autotuner for the mixed stage kernel: times configurations on the integrator's own buffers (a
+// realistic stage, CUDA events on the context stream, one warm and two timed launches each) and
+// keeps the fastest for this problem: by default the four-stage and eight-stage groups' large
+// tiles (on large grids; a rule picks them on small ones), with a group size or configuration
+// asked for all that match, with groups off every single-stage configuration.
 static void autotune_stage32(LSRKMem* m, STS_Problem p)
 {
   m->tuned       = true;
   m->tma_variant = -1;
   m->fuse_ks     = 1;
   m->fuse_ti     = -1;
+  m->deep_ti     = -1;
   if (m->stage_variant != 0 || !m->tma.ok) return;
+  const bool by_default = m->fuse_req == 0 && m->fuse_tile_req < 0 && m->tma.fz_ok && m->smax >= 9;
+  if (by_default && m->n < 10240LL * m->ctx->num_sms)
+  { // Grids below 1.6 million points: a launch is a chain of load, stages and barriers, and the
+    // shortest chain is the shortest tile that fits one wave (us per eight-stage launch with 16 /
+    // 32 / 48 rows: 128^2 8.3 / 10.4 / 10.7, 512^2 10.8 / 10.4 / 11.2, 1024 x 1500 25 / 22 / 23;
+    // per stage 1.0-2.8, four stages per launch 1.8-3.1). Timing all configurations costs 1.1 ms,
+    // as much as several steps on such a grid.
+    const long long sms = m->ctx->num_sms, cols = (p->nx + 111) / 112;
+    m->deep_ti     = cols * ((p->ny + 15) / 16) <= sms ? 8 : cols * ((p->ny + 31) / 32) <= 3 * sms * 11 / 10 ? 7 : 6;
+    m->fuse_ks     = 4;
+    m->fuse_ti     = 0;
+    m->tma_variant = 1;
+    return;
+  }
   cudaStream_t st = m->ctx->stream;
   // stage coefficients of a mid stage of a 100-stage RKL2 step (any finite values time alike)
   memset(m->h_par, 0, m->par_bytes);
@@ -645,23 +708,26 @@ static void autotune_stage32(LSRKMem* m, STS_Problem p)
   // scratch only: the stage buffers and the FP32 F of the other parity (the current one may
   // hold a restored or reset state)
   const int fpar = 1 - m->par;
-  cudaMemsetAsync(m->D[0], 0, m->n * sizeof(float), st);
-  cudaMemsetAsync(m->D[1], 0, m->n * sizeof(float), st);
-  cudaMemsetAsync(m->Ffb[fpar], 0, m->n * sizeof(float), st);
+  cudaMemsetAsync(m->D[0], 0, f32_field_bytes(m), st);
+  cudaMemsetAsync(m->D[1], 0, f32_field_bytes(m), st);
+  cudaMemsetAsync(m->Ffb[fpar], 0, f32_field_bytes(m), st);
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
   double best = 1e30;
-  for (int v = -1; v < TMA_STAGE32_NVARIANTS; ++v)
+  // (by default a single stage is the rest of a step at most, on the configuration that streams
+  // large grids fastest)
+  if (by_default) m->tma_variant = 4;
+  for (int v = -1; v < TMA_STAGE32_NVARIANTS && !by_default; ++v)
   {
-    for (int k = 0; k < 2; ++k) launch_stage32_idx(m, p, dstage(m) + 2, 0, 1, fpar, 2, v);
+    launch_stage32_idx(m, p, dstage(m) + 2, 0, 1, fpar, 2, v);
     cudaEventRecord(e0, st);
-    for (int k = 0; k < 5; ++k) launch_stage32_idx(m, p, dstage(m) + 2, 0, 1, fpar, 2, v);
+    for (int k = 0; k < 2; ++k) launch_stage32_idx(m, p, dstage(m) + 2, 0, 1, fpar, 2, v);
     cudaEventRecord(e1, st);
     if (cudaEventSynchronize(e1) != cudaSuccess) break;
     float ms = 0.f;
     cudaEventElapsedTime(&ms, e0, e1);
-    const double per = ms / 5.0;
+    const double per = ms / 2.0;
     m->tune_ms[v + 1] = per;
     if (per < best)
     {
@@ -676,23 +742,29 @@ static void autotune_stage32(LSRKMem* m, STS_Problem p)
   {
     for (int k = 3; k <= 5; ++k) hstage(m)[k] = *a;
     cudaMemcpyAsync(m->d_par, m->h_par, m->par_bytes, cudaMemcpyHostToDevice, st);
-    cudaMemsetAsync(m->D[2], 0, m->n * sizeof(float), st);
+    cudaMemsetAsync(m->D[2], 0, f32_field_bytes(m), st);
+    // milliseconds per launch of ks stages on a tile configuration
+    auto time_group = [&](int ti, int ks) {
+      auto one = [&]() {
+        return tma_fused_launch(&m->tma, ti, ks, m->ctx->num_sms, p->dev, dstage(m) + 2, 0, 1, fpar, m->D[2], m->D[3],
+                                m->ctx->d_err, st);
+      };
+      bool ok = one();
+      cudaEventRecord(e0, st);
+      for (int k = 0; k < 2 && ok; ++k) ok = one();
+      cudaEventRecord(e1, st);
+      float ms = -2.f;
+      if (ok && cudaEventSynchronize(e1) == cudaSuccess) cudaEventElapsedTime(&ms, e0, e1);
+      return ms / 2.0;
+    };
     double best_f = 1e30;
     for (int ti = 0; ti < TMA_FUSED_NTILES; ++ti)
     {
       if (m->fuse_tile_req >= 0 && ti != m->fuse_tile_req) continue;
-      auto one = [&]() {
-        return tma_fused_launch(&m->tma, ti, 4, m->ctx->num_sms, p->dev, dstage(m) + 2, 0, 1, fpar, m->D[2], m->D[3],
-                                m->ctx->d_err, st);
-      };
-      bool ok = one() && one();
-      cudaEventRecord(e0, st);
-      for (int k = 0; k < 5 && ok; ++k) ok = one();
-      cudaEventRecord(e1, st);
-      if (!ok || cudaEventSynchronize(e1) != cudaSuccess) break;
-      float ms = 0.f;
-      cudaEventElapsedTime(&ms, e0, e1);
-      m->fuse_ms[ti] = ms / 5.0;
+      if (by_default && ti != 1) continue; // 120 x 64, two CTAs per SM: within 2 % of the best on every large grid
+      const double per = time_group(ti, 4);
+      if (per < 0.0) break;
+      m->fuse_ms[ti] = per;
       if (m->fuse_ms[ti] < best_f)
       {
         best_f     = m->fuse_ms[ti];
@@ -703,6 +775,24 @@ static void autotune_stage32(LSRKMem* m, STS_Problem p)
     {
       if (m->fuse_req >= 2) m->fuse_ks = m->fuse_req;
       else if (best_f / 4.0 < best) m->fuse_ks = 4;
+    }
+    if (by_default && m->fuse_ks == 4)
+    { // eight stages per launch on tiles with a wider halo, where they are faster by more than the
+      // timing's noise (grids that stay in L2 gain nothing from less traffic)
+      for (int k = 6; k <= 9; ++k) hstage(m)[k] = *a;
+      cudaMemcpyAsync(m->d_par, m->h_par, m->par_bytes, cudaMemcpyHostToDevice, st);
+      double best_s = 0.97 * best_f / 4.0;
+      for (int ti = TMA_FUSED_NTILES; ti < TMA_FUSED_NALL - 1; ++ti) // (16 rows: small grids only)
+      {
+        const double per = time_group(ti, 8);
+        if (per < 0.0) break;
+        if (per / 8.0 < best_s)
+        {
+          best_s     = per / 8.0;
+          m->deep_ti = ti;
+          m->deep_ms = per;
+        }
+      }
     }
   }
   cudaEventDestroy(e0);
@@ -800,7 +890,7 @@ static void record_step(LSRKMem* m, STS_Problem p, int s, int par)
   }
   else
   {
-    stage1_32_kernel<<<eb, 256, 0, st>>>(n, dstep(m), m->Ffb[par], m->D[0]);
+    stage1_32_kernel<<<eb, 256, 0, st>>>(p->dev.ldf * p->ny, dstep(m), m->Ffb[par], m->D[0]);
     int im2 = -1, im1 = 0;
     const int nbuf = m->fuse_ks > 1 ? 4 : 3;
     auto free_buf = [&](int skip) { // a stage buffer that is neither input nor `skip`
@@ -810,14 +900,15 @@ static void record_step(LSRKMem* m, STS_Problem p, int s, int par)
     };
     for (int j = 2; j <= s;)
     {
-      const int ks = std::min(m->fuse_ks, s - j + 1);
+      const bool deep = m->deep_ti >= 0 && s - j + 1 >= 8;
+      const int ks    = deep ? 8 : std::min(m->fuse_ks, s - j + 1);
       if (ks >= 2)
       {
         // stages j .. j+ks-1 in one launch; the group's last two stages land in the two
         // buffers that are not its inputs
         const int o2 = free_buf(-1), o1 = free_buf(o2);
-        if (tma_fused_launch(&m->tma, m->fuse_ti, ks, m->ctx->num_sms, p->dev, dstage(m) + j, im1, im2, par,
-                             m->D[o2], m->D[o1], m->ctx->d_err, st))
+        if (tma_fused_launch(&m->tma, deep ? m->deep_ti : m->fuse_ti, ks, m->ctx->num_sms, p->dev, dstage(m) + j, im1,
+                             im2, par, m->D[o2], m->D[o1], m->ctx->d_err, st))
         {
           im2 = o2;
           im1 = o1;
@@ -1083,7 +1174,7 @@ static int evolve_fused(LSRKMem* m, double tout, double clip, int itask)
   {
     sts_rhs_launch(p, m->t, m->yb[m->par], m->Fb[m->par], true, st);
     m->nfe++;
-    if (m->mixed) sts_f64_to_f32(m->ctx, m->Fb[m->par], m->Ffb[m->par], n);
+    if (m->mixed) field_to_f32(m->ctx, p, m->Fb[m->par], m->Ffb[m->par]);
     m->hnext           = (m->hfixed > 0.0) ? m->hfixed : 0.0;
     m->initialized     = true;
     m->steps_since_dee = -1;
@@ -1793,7 +1884,10 @@ extern "C" int STS_LSRKStepGetStageKernelInfo(void* mem, int* variant, double* m
   if (name && namelen > 0)
   {
     const char* nm = m->mixed ? tma_stage32_variant_name(v) : "fp64_register_marching";
-    if (m->mixed && m->fuse_ks > 1)
+    if (m->mixed && m->deep_ti >= 0)
+      snprintf(name, namelen, "fused8_%s (rest: fused%d_%s)", tma_fused_config_name(m->deep_ti), m->fuse_ks,
+               tma_fused_config_name(m->fuse_ti));
+    else if (m->mixed && m->fuse_ks > 1)
       snprintf(name, namelen, "fused%d_%s (single stages: %s)", m->fuse_ks, tma_fused_config_name(m->fuse_ti), nm);
     else snprintf(name, namelen, "%s", nm);
   }
@@ -1823,6 +1917,14 @@ extern "C" int STS_LSRKStepGetStageFusion(void* mem, int* ks, int* config, int* 
 {
   CHECK_MEM(mem);
   LSRKMem* m = MEM(mem);
+  if (m->mixed && m->deep_ti >= 0)
+  {
+    if (ks) *ks = 8;
+    if (config) *config = m->deep_ti + 1;
+    if (tile_rows) *tile_rows = tma_fused_tile_rows(m->deep_ti);
+    if (ms_per_launch) *ms_per_launch = m->deep_ms;
+    return 0;
+  }
   const bool on = m->mixed && m->fuse_ks > 1;
   if (ks) *ks = on ? m->fuse_ks : 1;
   if (config) *config = on ? m->fuse_ti + 1 : 0;
@@ -1980,7 +2082,7 @@ extern "C" int STS_ARKodeReset(void* mem, double t, N_Vector y)
     {
       STS_Problem p = (STS_Problem)m->user_data;
       sts_rhs_launch(p, m->t, m->yb[m->par], m->Fb[m->par], true, m->ctx->stream);
-      if (m->mixed) sts_f64_to_f32(m->ctx, m->Fb[m->par], m->Ffb[m->par], m->n);
+      if (m->mixed) field_to_f32(m->ctx, p, m->Fb[m->par], m->Ffb[m->par]);
     }
     else if (m->rhs(m->t, m->g_y, m->g_Fn, m->user_data) != 0)
       return STS_RHSFUNC_FAIL;
@@ -2003,11 +2105,12 @@ extern "C" int STS_LSRKStepTimeStageKernel(void* mem, int nlaunch, double* ms_pe
   cudaEventCreate(&e1);
   // the parameter block of the last step is still on the device
   // fused stages: one launch of the step's stage groups (stages j .. j+ks-1)
-  const int ks = (m->mixed && m->fuse_ks > 1 && m->last_s >= m->fuse_ks + 1) ? m->fuse_ks : 1;
+  const int kw = m->deep_ti >= 0 && m->last_s >= 9 ? 8 : m->fuse_ks;
+  const int ks = (m->mixed && kw > 1 && m->last_s >= kw + 1) ? kw : 1;
   const int jf = (ks > 1 && j + ks - 1 > m->last_s) ? 2 : j;
   auto one = [&](int k) {
     if (ks > 1)
-      tma_fused_launch(&m->tma, m->fuse_ti, ks, m->ctx->num_sms, p->dev, dstage(m) + jf, k % 4, (k + 1) % 4, m->par,
+      tma_fused_launch(&m->tma, ks == 8 ? m->deep_ti : m->fuse_ti, ks, m->ctx->num_sms, p->dev, dstage(m) + jf, k % 4, (k + 1) % 4, m->par,
                        m->D[(k + 2) % 4], m->D[(k + 3) % 4], m->ctx->d_err, st);
     else if (m->mixed) launch_stage32_idx(m, p, dstage(m) + j, k % 3, (k + 1) % 3, m->par, (k + 2) % 3);
     else launch_stage64(m, p, dstage(m) + j, m->Y[k % 3], m->Y[(k + 1) % 3], m->yb[m->par], m->Fb[m->par], m->Y[(k + 2) % 3]);
@@ -2097,6 +2200,24 @@ void sts_f64_to_f32(STS_Context ctx, const double* a, float* b, long long n)
   f64_to_f32_kernel<<<ew_blocks(ctx, n, 256 * 4), 256, 0, ctx->stream>>>(n, a, b);
 }
 
+// the FP32 copy of a field, rows padded to ProbDev::ldf
+__global__ void field_to_f32_kernel(ProbDev P, const double* __restrict__ a, float* __restrict__ b)
+{
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= P.nx) return;
+  for (long long j = blockIdx.y; j < P.ny; j += gridDim.y) b[j * P.ldf + i] = (float)a[j * P.nx + i];
+}
+
+static void field_to_f32(STS_Context ctx, STS_Problem p, const double* a, float* b)
+{
+  if (p->dev.ldf == p->nx) sts_f64_to_f32(ctx, a, b, p->nx * p->ny);
+  else
+  {
+    const dim3 g((unsigned)((p->nx + 255) / 256), (unsigned)std::min<long long>(p->ny, 65535));
+    field_to_f32_kernel<<<g, 256, 0, ctx->stream>>>(p->dev, a, b);
+  }
+}
+
 void sts_hermite_coeffs(int deg, double tau, double h, double a[4])
 {
   const double tau2 = tau * tau, tau3 = tau * tau2;
@@ -2182,6 +2303,18 @@ static bool ckpt_io(FILE* f, void* host, const void* dev, void* dev_out, size_t 
          STS_CUDA_OK(cudaStreamSynchronize(st));
 }
 
+// the FP32 copy of F_n: in the file without the rows' padding
+static bool ckpt_io_f32(FILE* f, void* host, STS_Problem p, float* dev, bool write, cudaStream_t st)
+{
+  const size_t row = p->nx * sizeof(float), pitch = p->dev.ldf * sizeof(float), bytes = row * p->ny;
+  if (!write && fread(host, 1, bytes, f) != bytes) return false;
+  if (!STS_CUDA_OK(write ? cudaMemcpy2DAsync(host, row, dev, pitch, row, p->ny, cudaMemcpyDeviceToHost, st)
+                         : cudaMemcpy2DAsync(dev, pitch, host, row, row, p->ny, cudaMemcpyHostToDevice, st)) ||
+      !STS_CUDA_OK(cudaStreamSynchronize(st)))
+    return false;
+  return !write || fwrite(host, 1, bytes, f) == bytes;
+}
+
 extern "C" int STS_LSRKStepWriteCheckpoint(void* mem, const char* path)
 {
   CHECK_MEM(mem);
@@ -2234,7 +2367,7 @@ extern "C" int STS_LSRKStepWriteCheckpoint(void* mem, const char* path)
   ok = ok && ckpt_io(f, host.data(), y, nullptr, m->n * sizeof(double), true, st);
   if (m->initialized) ok = ok && ckpt_io(f, host.data(), F, nullptr, m->n * sizeof(double), true, st);
   if (m->initialized && fz && m->mixed)
-    ok = ok && ckpt_io(f, host.data(), m->Ffb[m->par], nullptr, m->n * sizeof(float), true, st);
+    ok = ok && ckpt_io_f32(f, host.data(), (STS_Problem)m->user_data, m->Ffb[m->par], true, st);
   if (h.has_evec) ok = ok && ckpt_io(f, host.data(), m->evec, nullptr, m->n * sizeof(double), true, st);
   ok = (fclose(f) == 0) && ok;
   if (!ok) sts_set_error("STS_LSRKStepWriteCheckpoint: write to %s failed", path);
@@ -2283,7 +2416,7 @@ extern "C" int STS_LSRKStepReadCheckpoint(void* mem, const char* path)
   ok = ckpt_io(f, host.data(), nullptr, y, m->n * sizeof(double), false, st);
   if (h.initialized) ok = ok && ckpt_io(f, host.data(), nullptr, F, m->n * sizeof(double), false, st);
   if (h.initialized && fz && h.mixed)
-    ok = ok && ckpt_io(f, host.data(), nullptr, m->Ffb[0], m->n * sizeof(float), false, st);
+    ok = ok && ckpt_io_f32(f, host.data(), (STS_Problem)m->user_data, m->Ffb[0], false, st);
   if (ok && h.has_evec)
   {
     if (!m->evec && !STS_CUDA_OK(cudaMalloc(&m->evec, m->n * sizeof(double)))) ok = false;

@@ -157,8 +157,9 @@ __global__ void __launch_bounds__(256, K::MINB)
         o[v] = mixed_point<FORCED>(gs, gx, gy, gm, gF, cv[v], uw, ue, uv[v], dv[v], mv[v], qv[v], syj, Pi[v], syyj,
                                    Qi[v]);
       }
-      if (y < ny && x < nx && STS_IN_BOUNDS(x + 4 <= nx, err))
-        *reinterpret_cast<float4*>(out + (long long)y * nx + x) = make_float4(o[0], o[1], o[2], o[3]);
+      // (a row's last quad may reach into its padding, which no copy reads)
+      if (y < ny && x < nx && STS_IN_BOUNDS(x + 4 <= P.ldf, err))
+        *reinterpret_cast<float4*>(out + (long long)y * P.ldf + x) = make_float4(o[0], o[1], o[2], o[3]);
       up  = cur;
       cur = dn;
     }
@@ -210,7 +211,7 @@ bool encode(CUtensorMap* m, const float* base, long long nx, long long ny, int b
   EncodeTiledFn fn = encode_fn();
   if (!fn) return false;
   cuuint64_t dims[2]    = {(cuuint64_t)nx, (cuuint64_t)ny};
-  cuuint64_t strides[1] = {(cuuint64_t)nx * 4};
+  cuuint64_t strides[1] = {(cuuint64_t)((nx + 3) / 4 * 4) * 4}; // ProbDev::ldf
   cuuint32_t box[2]     = {(cuuint32_t)bw, (cuuint32_t)bh};
   cuuint32_t es[2]      = {1, 1};
   CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, (void*)base, dims, strides, box, es,
@@ -279,9 +280,9 @@ bool tma_encode_f32_2d(CUtensorMap* m, const float* base, long long nx, long lon
 
 bool tma_stage32_supported(long long nx, long long ny)
 {
-  // 16-byte row pitch and 16-byte aligned x coordinates (multiples of 4 floats); the tile
-  // coordinates must fit the copy engine's signed 32-bit coordinates
-  return nx % 4 == 0 && nx >= 8 && ny >= 2 && nx < (1LL << 30) && ny < (1LL << 30) && encode_fn() != nullptr;
+  // the row pitch (ProbDev::ldf) and the x coordinates are multiples of 4 floats for every nx; the
+  // tile coordinates must fit the copy engine's signed 32-bit coordinates
+  return nx >= 8 && ny >= 2 && nx < (1LL << 30) && ny < (1LL << 30) && encode_fn() != nullptr;
 }
 
 bool tma_stage32_prepare(TmaStage32* t, float* const D[4], float* const Ff[2], long long nx, long long ny)

@@ -195,6 +195,7 @@ __device__ __forceinline__ void xsum_block_finish(xsum::Limbs& a, unsigned flags
 // ---------------------------------------------------------------------------------------
 struct ProbDev {
   long long nx, ny;
+  long long ldf; // row pitch of the mixed form's FP32 fields: nx rounded up to 4 (16-byte rows)
   int kind, inhom;
   double kx, ky, cx, cy, cc;
   const double *Sx, *Sxx, *Sy, *Syy;

@@ -244,24 +244,24 @@ int STS_ARKodeSetMaxNumSteps(void* mem, long long mxsteps);           /* main.cp
 int STS_ARKodeSetStopTime(void* mem, double tstop);                   /* main.cpp:384 */
 /* new: FP32 stage increments relative to the FP64 step-start state (fused path only) */
 int STS_LSRKStepSetMixedPrecision(void* mem, int on);
-/* new: mixed-stage kernel selection: 0 = autotuned at the first step among the TMA +
- * mbarrier pipelined tile configurations (rows per tile, ring depth, CTAs per SM; row length
- * a multiple of 4) and the register-marching kernel (default), 1 = register-marching kernel,
+/* new: mixed-stage kernel selection: 0 = chosen at the first step (with stage groups off: timed) among the TMA +
+ * mbarrier pipelined tile configurations (rows per tile, ring depth, CTAs per SM) and the register-marching kernel (default), 1 = register-marching kernel,
  * 2 + k = TMA configuration k (k < 6). All variants give identical bits. */
 int STS_LSRKStepSetStageKernel(void* mem, int variant);
 /* new: the autotuner's choice (-1 = register-marching), its time per launch and its name */
 int STS_LSRKStepGetStageKernelInfo(void* mem, int* variant, double* ms_per_launch, char* name,
                                    int namelen);
 /* new: mixed form, several stages per launch (temporal blocking on 120-column tiles in shared
-   memory, the same bits as one launch per stage). ks: 0 = autotuned (default: four stages per
-   launch when the autotuner times that faster than one), 1 = off, 2..4 = that many; config:
-   0 = autotuned, 1..6 = tile configuration (1: 120 x 32, three CTAs per SM; 2, 3, 5: 120 x 64,
+   memory, the same bits as one launch per stage). ks: 0 = autotuned (default: eight or four
+   stages per launch when the autotuner times that faster than one; eight, untimed, below 1.6
+   million points), 1 = off, 2..4 = that many;
+   config: 0 = autotuned, 1..6 = tile configuration (1: 120 x 32, three CTAs per SM; 2, 3, 5: 120 x 64,
    120 x 60 and 120 x 58, two CTAs of 256 threads per SM; 4: 120 x 64, two CTAs of 384 threads;
    6: 120 x 64, one CTA of 256 threads per SM with two tile buffers).
    Applies with the autotuned stage kernel (STS_LSRKStepSetStageKernel variant 0). */
 int STS_LSRKStepSetStageFusion(void* mem, int ks, int config);
-/* new: the stages per launch in use (1: none), the tile configuration (0: none) and its rows,
-   and the autotuner's time per four-stage launch */
+/* new: the stages per launch in use (1: none), the tile configuration (0: none; above 6: the
+   112-column tiles of the eight-stage groups) and its rows, and the autotuner's time per launch */
 int STS_LSRKStepGetStageFusion(void* mem, int* ks, int* config, int* tile_rows, double* ms_per_launch);
 /* new: capture the fixed-s stage loop of the fused path in CUDA graphs (default on) */
 int STS_LSRKStepSetUseGraphs(void* mem, int on);

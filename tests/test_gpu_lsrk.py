@@ -531,3 +531,34 @@ def test_fp64_stage_rows_per_thread_bitwise(ctx, stslib, oracle, nx, ny, kind):
     assert J.evolve(h) == 0
     assert I.stats()["nst"] == 1 and I.stats()["stage_max"] >= 5
     assert np.array_equal(y.numpy(), J.y)
+
+
+@pytest.mark.parametrize("nx,ny", [(9, 40), (111, 17), (112, 16), (113, 15), (226, 49), (337, 33), (1021, 50)])
+@pytest.mark.parametrize("kind", [0, 1])
+def test_mixed_default_groups_on_odd_rows_bitwise(ctx, stslib, oracle, tmp_path, nx, ny, kind):
+    """The mixed form's autotuned default (groups of eight stages on 112-column tiles, the rest of a
+    step in groups of four) on rows that no vector width divides, one column and one row around
+    the tile edges, forced and unforced, against the oracle; a checkpoint (it holds the FP32 copy
+    of F_n without the rows' padding) read into a new integrator continues with the same bits."""
+    pk = dict(kind=kind, nx=nx, ny=ny, kx=0.5 * (300.0 / max(nx, ny)) ** 2, ky=0.01)
+    modes = (np.array([1, 3]), np.array([2, 1]), np.array([1.0, -0.5]))
+    ok = dict(method=1, rtol=1e-3, atol=1e-6, mixed=True)
+    G, O = stslib.Problem(ctx, **pk), oracle.Problem(**pk)
+    y0, yo = (G.initial(), O.initial()) if kind == 0 else (G.initial_modes(*modes), O.initial_modes(*modes))
+    I = stslib.LSRKStep(ctx, G, 0.0, y0, **ok)
+    J = oracle.Integrator(O, yo, **ok)
+    y = G.vector()
+    I.evolve(0.01, y)
+    assert J.evolve(0.01) == 0
+    so, sg = J.stats(), I.stats()
+    assert kind or so["stage_max"] >= 9
+    assert all(sg[k] == so[k] for k in STAT_KEYS)
+    assert np.array_equal(y.numpy(), J.y)
+    I.write_checkpoint(str(tmp_path / "state.ckpt"))
+    K = stslib.LSRKStep(ctx, G, 0.0, y0, **ok)
+    K.read_checkpoint(str(tmp_path / "state.ckpt"))
+    z = G.vector()
+    t2 = 2.0 * sg["t"]  # past the last step: a new integrator holds no step to interpolate on
+    I.evolve(t2, y)
+    K.evolve(t2, z)
+    assert np.array_equal(y.numpy(), z.numpy()) and I.stats()["nst"] == K.stats()["nst"]
