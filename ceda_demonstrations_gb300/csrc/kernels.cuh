@@ -125,7 +125,7 @@ __device__ __forceinline__ double mixed_weight(double rtol, double atol, double 
   const long long u = __double_as_longlong(den);
   if (u >= 0x3870000000000000LL && u <= 0x4770000000000000LL)
   {
-    const double r0 = (double)__frcp_rn(__double2float_rn(den));
+    const double r0 = s64_from_float(__frcp_rn(s64_to_float(den)));
     const double e1 = __fma_rn(-den, r0, 1.0);
     return __fma_rn(r0, e1, r0);
   }
@@ -340,12 +340,17 @@ static __global__ void __launch_bounds__(256) stage1_32_kernel(long long n, cons
 // ---------------------------------------------------------------------------------------
 // Step end. Fnew = F(t+h, ynew); err = 0.8 (yn - ynew) + 0.4 h (Fn + Fnew);
 // dsm = sqrt(sum (err/(rtol |yn| + atol))^2 / N) with the exact accumulator.
-// MIXED: ynew = yn + (double) ds is formed on the fly (also at the stencil neighbours) and
-// written out together with Fnew and its FP32 copy; yn - ynew is taken as -ds and the weight
-// comes from mixed_weight.
-// Grid: blockDim.x columns per block, blocks stride over rows.
+// MIXED: ynew = yn + (double) ds is formed on the fly (once per point; the west/east neighbours
+// come from the neighbouring lanes, lanes 0 and 31 form the one they lack) and written out
+// together with Fnew and its FP32 copy; yn - ynew is taken as -ds and the weight comes from
+// mixed_weight. A thread owns one column and RY rows, rows j-1, j, j+1 of ynew in registers.
+//
+// Bound by the FP64 pipe: in the mixed form 21 FP64 instructions per point, of which the four
+// products, the neighbour sums and the conversions between the formats (which take the FP64 pipe
+// too) are integer code here (soft64.cuh), about 11 are left: 2.9 -> 2.1 ms at 8192^2 forced. On
+// small grids the rows of a thread and the reduction's tail set the time (launch_stepend).
 // ---------------------------------------------------------------------------------------
-template <bool MIXED, bool FORCED>
+template <int RY, bool MIXED, bool FORCED>
 __global__ void __launch_bounds__(256) stepend_kernel(ProbDev P, const StepArgs* __restrict__ S,
                                                       const double* __restrict__ yn,
                                                       const double* __restrict__ Ys,
@@ -358,204 +363,83 @@ __global__ void __launch_bounds__(256) stepend_kernel(ProbDev P, const StepArgs*
 {
   const long long nx = P.nx, ny = P.ny;
   const long long i  = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const long long jb = ((long long)blockIdx.y * blockDim.y + threadIdx.y) * RY;
+  const int lane     = threadIdx.x & 31;
   const double p4h = S->p4h, rtol = S->rtol, atol = S->atol;
-  const double al = S->al, be = S->be, ga = S->ga;
+  const soft64::Factor ccF = soft64::factor(P.cc), c8F = soft64::factor(0.8);
   xsum::Limbs acc;
   xsum::zero(acc);
   unsigned flags = 0;
-  if (i < nx)
+  // no early return: the shuffles and the block reduction below take every thread
+  const bool active = i < nx && jb < ny && STS_IN_BOUNDS(jb * nx + i < nx * ny, P.err);
+  // y_{n+1} at (i, j), zero outside the domain
+  auto point = [&](long long ii, long long j) -> double {
+    if (ii < 0 || ii >= nx || j < 0 || j >= ny) return 0.0;
+    if (MIXED) return __ldg(yn + j * nx + ii) + s64_from_float(__ldg(ds + j * P.ldf + ii));
+    return __ldg(Ys + j * nx + ii);
+  };
+  double Pi = 0.0, Qi = 0.0;
+  if (FORCED && active)
   {
-    double Pi = 0.0, Qi = 0.0;
-    if (FORCED)
-    {
-      Pi = __fma_rn(al, P.Sx[i], be * P.Sxx[i]);
-      Qi = ga * P.Sx[i];
-    }
-    for (long long j = blockIdx.y; j < ny; j += gridDim.y)
-    {
-      const long long k = j * nx + i, kf = j * P.ldf + i;
-      double uc, uw, ue, us, un;
-      if (MIXED)
-      {
-        uc = yn[k] + (double)ds[kf];
-        uw = (i > 0) ? yn[k - 1] + (double)ds[kf - 1] : 0.0;
-        ue = (i < nx - 1) ? yn[k + 1] + (double)ds[kf + 1] : 0.0;
-        us = (j > 0) ? yn[k - nx] + (double)ds[kf - P.ldf] : 0.0;
-        un = (j < ny - 1) ? yn[k + nx] + (double)ds[kf + P.ldf] : 0.0;
-      }
-      else
-      {
-        uc = Ys[k];
-        uw = (i > 0) ? Ys[k - 1] : 0.0;
-        ue = (i < nx - 1) ? Ys[k + 1] : 0.0;
-        us = (j > 0) ? Ys[k - nx] : 0.0;
-        un = (j < ny - 1) ? Ys[k + nx] : 0.0;
-      }
-      const double sx = uw + ue, sy = us + un;
-      double f        = P.cc * uc;
-      f               = __fma_rn(P.cx, sx, f);
-      f               = __fma_rn(P.cy, sy, f);
-      if (FORCED)
-      {
-        f = __fma_rn(P.Sy[j], Pi, f);
-        f = __fma_rn(P.Syy[j], Qi, f);
-      }
-      Fnew[k] = f;
-      if (MIXED)
-      {
-        ynew[k]  = uc;
-        Fnewf[kf] = (float)f;
-      }
-      const double y = yn[k];
-      // the mixed form takes y_n - y_{n+1} as -d_s itself (exact) and the fast weight
-      const double d = MIXED ? -(double)ds[kf] : y - uc;
-      double e       = 0.8 * d;
-      e              = __fma_rn(p4h, Fn[k], e);
-      e              = __fma_rn(p4h, f, e);
-      const double wt = MIXED ? mixed_weight(rtol, atol, y) : 1.0 / (rtol * fabs(y) + atol);
-      const double x  = e * wt;
-      xsum::add(acc, x * x, flags);
-    }
+    Pi = __fma_rn(S->al, P.Sx[i], S->be * P.Sxx[i]);
+    Qi = S->ga * P.Sx[i];
   }
-  xsum_block_finish<256>(acc, flags, w, slot, 1, (double)(nx * ny));
-}
-
-// Step end, row-marching form (nx even): a thread owns 2 consecutive columns and 16 rows,
-// keeps rows j-1, j, j+1 of y_{n+1} in registers (formed once per point, yn + ds in the
-// mixed form), and gets the west/east neighbours from the neighbouring lanes; per point the
-// arithmetic is identical to stepend_kernel.
-template <bool MIXED, bool FORCED>
-__global__ void __launch_bounds__(256) stepend_march_kernel(ProbDev P, const StepArgs* __restrict__ S,
-                                                            const double* __restrict__ yn,
-                                                            const double* __restrict__ Ys,
-                                                            const float* __restrict__ ds,
-                                                            const double* __restrict__ Fn,
-                                                            double* __restrict__ ynew,
-                                                            double* __restrict__ Fnew,
-                                                            float* __restrict__ Fnewf, RedWork* w,
-                                                            double* slot)
-{
-  constexpr int RYS = 16;
-  const long long nx = P.nx, ny = P.ny;
-  const long long i0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * 2;
-  const long long jb = ((long long)blockIdx.y * blockDim.y + threadIdx.y) * RYS;
-  const int lane     = threadIdx.x & 31;
-  const double p4h = S->p4h, rtol = S->rtol, atol = S->atol;
-  xsum::Limbs acc;
-  xsum::zero(acc);
-  unsigned flags   = 0;
-  const bool colok = i0 < nx; // nx even: both columns valid
-  // no early return here: the block reduction below has barriers
-  const bool active = colok && jb < ny && STS_IN_BOUNDS(i0 + 2 <= nx, P.err);
-  // y_{n+1} at (row, i0..i0+1); zero outside the domain
-  auto row2 = [&](long long j, double (&v)[2]) {
-    if (!active || j < 0 || j >= ny)
-    {
-      v[0] = v[1] = 0.0;
-      return;
-    }
-    const long long k = j * nx + i0;
+  double up = active ? point(i, jb - 1) : 0.0, cur = active ? point(i, jb) : 0.0;
+#pragma unroll 1
+  for (int r = 0; r < RY; ++r)
+  {
+    const long long j = jb + r;
+    const bool row    = active && j < ny;
+    const double dn   = row ? point(i, j + 1) : 0.0;
+    double uw, ue;
     if (MIXED)
     {
-      const double2 a = __ldg(reinterpret_cast<const double2*>(yn + k));
-      const float2 b  = __ldg(reinterpret_cast<const float2*>(ds + j * P.ldf + i0));
-      v[0]            = a.x + (double)b.x;
-      v[1]            = a.y + (double)b.y;
+      uw = __shfl_up_sync(0xffffffffu, cur, 1);
+      ue = __shfl_down_sync(0xffffffffu, cur, 1);
+      if (row && (lane == 0 || lane == 31))
+      {
+        const double o = point(lane == 0 ? i - 1 : i + 1, j);
+        if (lane == 0) uw = o;
+        else ue = o;
+      }
+      if (i + 1 >= nx) ue = 0.0;
     }
     else
     {
-      const double2 a = __ldg(reinterpret_cast<const double2*>(Ys + k));
-      v[0]            = a.x;
-      v[1]            = a.y;
+      uw = row ? point(i - 1, j) : 0.0;
+      ue = row ? point(i + 1, j) : 0.0;
     }
-  };
-  auto point = [&](long long j, long long i) -> double { // single y_{n+1} value (edges)
-    if (i < 0 || i >= nx || j < 0 || j >= ny) return 0.0;
-    const long long k = j * nx + i;
-    return MIXED ? yn[k] + (double)ds[j * P.ldf + i] : Ys[k];
-  };
-  double Pi[2] = {0.0, 0.0}, Qi[2] = {0.0, 0.0};
-  if (FORCED && colok)
-  {
-    const double al = S->al, be = S->be, ga = S->ga;
-#pragma unroll
-    for (int v = 0; v < 2; ++v)
+    if (row)
     {
-      Pi[v] = __fma_rn(al, P.Sx[i0 + v], be * P.Sxx[i0 + v]);
-      Qi[v] = ga * P.Sx[i0 + v];
-    }
-  }
-  double up[2], cur[2], dn[2];
-  row2(jb - 1, up);
-  row2(jb, cur);
-  for (int r = 0; r < RYS; ++r)
-  {
-    const long long j = jb + r;
-    row2(j + 1, dn);
-    // west/east neighbours from the neighbouring lanes (the warp spans 64 consecutive columns)
-    double wv = __shfl_up_sync(0xffffffffu, cur[1], 1);
-    double ev = __shfl_down_sync(0xffffffffu, cur[0], 1);
-    if (lane == 0) wv = active && j < ny ? point(j, i0 - 1) : 0.0;
-    if (lane == 31) ev = active && j < ny ? point(j, i0 + 2) : 0.0;
-    if (active && j < ny)
-    {
-      if (i0 + 2 >= nx) ev = 0.0;
-      if (i0 == 0) wv = 0.0;
-      const long long k = j * nx + i0;
-      const double2 ynv = __ldg(reinterpret_cast<const double2*>(yn + k));
-      const double2 fnv = __ldg(reinterpret_cast<const double2*>(Fn + k));
-      const double yv[2] = {ynv.x, ynv.y}, fv[2] = {fnv.x, fnv.y};
-      float dsv[2] = {0.f, 0.f};
-      if (MIXED)
-      {
-        const float2 t = __ldg(reinterpret_cast<const float2*>(ds + j * P.ldf + i0));
-        dsv[0]         = t.x;
-        dsv[1]         = t.y;
-      }
-      double syj = 0.0, syyj = 0.0;
+      const long long k = j * nx + i, kf = j * P.ldf + i;
+      double f = s64_mul(ccF, P.cc, cur);
+      f        = __fma_rn(P.cx, s64_add(uw, ue), f);
+      f        = __fma_rn(P.cy, s64_add(up, dn), f);
       if (FORCED)
       {
-        syj  = P.Sy[j];
-        syyj = P.Syy[j];
+        f = __fma_rn(__ldg(P.Sy + j), Pi, f);
+        f = __fma_rn(__ldg(P.Syy + j), Qi, f);
       }
-      double fo[2];
-#pragma unroll
-      for (int v = 0; v < 2; ++v)
-      {
-        const double uc = cur[v];
-        const double uw = (v == 0) ? wv : cur[0];
-        const double ue = (v == 1) ? ev : cur[1];
-        const double sx = uw + ue, sy = up[v] + dn[v];
-        double f        = P.cc * uc;
-        f               = __fma_rn(P.cx, sx, f);
-        f               = __fma_rn(P.cy, sy, f);
-        if (FORCED)
-        {
-          f = __fma_rn(syj, Pi[v], f);
-          f = __fma_rn(syyj, Qi[v], f);
-        }
-        fo[v]           = f;
-        const double d  = MIXED ? -(double)dsv[v] : yv[v] - uc;
-        double e        = 0.8 * d;
-        e               = __fma_rn(p4h, fv[v], e);
-        e               = __fma_rn(p4h, f, e);
-        const double wt = MIXED ? mixed_weight(rtol, atol, yv[v]) : 1.0 / (rtol * fabs(yv[v]) + atol);
-        const double x  = e * wt;
-        xsum::add(acc, x * x, flags);
-      }
-      *reinterpret_cast<double2*>(Fnew + k) = make_double2(fo[0], fo[1]);
+      Fnew[k] = f;
+      const double y = __ldg(yn + k);
+      double d;
       if (MIXED)
       {
-        *reinterpret_cast<double2*>(ynew + k) = make_double2(cur[0], cur[1]);
-        *reinterpret_cast<float2*>(Fnewf + j * P.ldf + i0) = make_float2((float)fo[0], (float)fo[1]);
+        ynew[k]   = cur;
+        Fnewf[kf] = s64_to_float(f);
+        // the mixed form takes y_n - y_{n+1} as -d_s itself (exact) and the fast weight
+        d = s64_from_float(-__ldg(ds + kf));
       }
+      else d = y - cur;
+      double e = s64_mul(c8F, 0.8, d);
+      e        = __fma_rn(p4h, __ldg(Fn + k), e);
+      e        = __fma_rn(p4h, f, e);
+      const double wt = MIXED ? mixed_weight(rtol, atol, y) : 1.0 / (rtol * fabs(y) + atol);
+      const double x  = s64_mul(e, wt);
+      xsum::add(acc, s64_mul(x, x), flags);
     }
-#pragma unroll
-    for (int v = 0; v < 2; ++v)
-    {
-      up[v]  = cur[v];
-      cur[v] = dn[v];
-    }
+    up  = cur;
+    cur = dn;
   }
   xsum_block_finish<256>(acc, flags, w, slot, 1, (double)(nx * ny));
 }

@@ -819,42 +819,41 @@ static void launch_stage32(LSRKMem* m, STS_Problem p, const StageArgs* A, const 
   else go(std::integral_constant<int, 1>{});
 }
 
+// Rows per thread of the step end by the rule of launch_stage64. Measured us per step of four
+// stages with 1 / 2 / 4 / 16 rows (before: 2 columns x 16 rows per thread): FP64 128^2 29 / 31 /
+// 35 / 54 (108), 512^2 52 / 51 / 51 / 69 (112), 1024^2 112 / 107 / 105 / 113 (145), 4096^2 1584 /
+// 1453 / 1384 / 1354 (1867); mixed 128^2 25 / 28 / 32 / 56 (78), 8192^2 4025 / 3162 / 2894 / 2688
+// (3525).
 static void launch_stepend(LSRKMem* m, STS_Problem p, int par, const double* Ys, const float* ds)
 {
   const bool forced = p->kind == STS_PROBLEM_MANUFACTURED;
-  if (p->nx % 2 == 0)
-  { // row-marching form: 64 x 4 threads, 2 columns x 16 rows each
-    dim3 b(64, 4);
-    dim3 g((unsigned)((p->nx / 2 + 63) / 64), (unsigned)((p->ny + 63) / 64));
-    const int nxt = 1 - par;
-    RedWork* w    = m->ctx->d_work;
-    double* slot  = m->ctx->d_slots + SLOT_DSM;
+  const int nxt     = 1 - par;
+  auto go = [&](auto Rc) {
+    constexpr int R = decltype(Rc)::value;
+    const dim3 b(64, 4);
+    const dim3 g((unsigned)((p->nx + b.x - 1) / b.x), (unsigned)((p->ny + b.y * R - 1) / (b.y * R)));
     dispatch_forced(forced, [&](auto F) {
       if (m->mixed)
-        stepend_march_kernel<true, decltype(F)::value><<<g, b, 0, m->ctx->stream>>>(
-          p->dev, dstep(m), m->yb[par], nullptr, ds, m->Fb[par], m->yb[nxt], m->Fb[nxt], m->Ffb[nxt], w, slot);
+        stepend_kernel<R, true, decltype(F)::value><<<g, b, 0, m->ctx->stream>>>(
+          p->dev, dstep(m), m->yb[par], nullptr, ds, m->Fb[par], m->yb[nxt], m->Fb[nxt], m->Ffb[nxt], m->ctx->d_work,
+          m->ctx->d_slots + SLOT_DSM);
       else
-        stepend_march_kernel<false, decltype(F)::value><<<g, b, 0, m->ctx->stream>>>(
-          p->dev, dstep(m), m->yb[par], Ys, nullptr, m->Fb[par], nullptr, m->Fb[nxt], nullptr, w, slot);
+        stepend_kernel<R, false, decltype(F)::value><<<g, b, 0, m->ctx->stream>>>(
+          p->dev, dstep(m), m->yb[par], Ys, nullptr, m->Fb[par], nullptr, m->Fb[nxt], nullptr, m->ctx->d_work,
+          m->ctx->d_slots + SLOT_DSM);
     });
-    return;
+  };
+  const long long n = p->nx * p->ny, W = 1024LL * m->ctx->num_sms;
+  const long long nyb = p->ny / (4 * 65535);
+  int rows = n < W ? 1 : n < 3 * W ? 2 : n < 10 * W ? 4 : 16;
+  while (rows < 16 && nyb >= rows) rows *= rows < 4 ? 2 : 4;
+  switch (rows)
+  {
+  case 1: go(std::integral_constant<int, 1>{}); break;
+  case 2: go(std::integral_constant<int, 2>{}); break;
+  case 4: go(std::integral_constant<int, 4>{}); break;
+  default: go(std::integral_constant<int, 16>{});
   }
-  dim3 b(256, 1);
-  unsigned gx      = (unsigned)((p->nx + 255) / 256);
-  long long gy_cap = std::max<long long>(1, (long long)m->ctx->num_sms * 8 / gx);
-  unsigned gy      = (unsigned)std::min<long long>(p->ny, gy_cap);
-  dim3 g(gx, gy);
-  const int nxt = 1 - par;
-  RedWork* w    = m->ctx->d_work;
-  double* slot  = m->ctx->d_slots + SLOT_DSM;
-  dispatch_forced(forced, [&](auto F) {
-    if (m->mixed)
-      stepend_kernel<true, decltype(F)::value><<<g, b, 0, m->ctx->stream>>>(
-        p->dev, dstep(m), m->yb[par], nullptr, ds, m->Fb[par], m->yb[nxt], m->Fb[nxt], m->Ffb[nxt], w, slot);
-    else
-      stepend_kernel<false, decltype(F)::value><<<g, b, 0, m->ctx->stream>>>(
-        p->dev, dstep(m), m->yb[par], Ys, nullptr, m->Fb[par], nullptr, m->Fb[nxt], nullptr, w, slot);
-  });
 }
 
 // Record the whole step (parameter upload, s stages, step end) on the stream. Buffers

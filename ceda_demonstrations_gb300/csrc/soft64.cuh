@@ -158,6 +158,44 @@ S64_HD bool fma_small(const Factor& f, double b, double c, double* r)
   return true;
 }
 
+S64_HD uint32_t bits32(float x)
+{
+#ifdef __CUDA_ARCH__
+  return (uint32_t)__float_as_int(x);
+#else
+  uint32_t b;
+  std::memcpy(&b, &x, 4);
+  return b;
+#endif
+}
+
+// (double)x: a normal x
+S64_HD bool from_float(float x, double* d)
+{
+  const uint32_t b = bits32(x);
+  if (((b >> 23) & 0xffu) - 1u > 253u) return false;
+  *d = value((b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + (896u << 20)), b << 29);
+  return true;
+}
+
+// (float)x, ties to even: x in the float format's normal range (a round up past it gives
+// infinity, as the conversion does)
+S64_HD bool to_float(double x, float* f)
+{
+  const uint64_t B  = bits(x);
+  const uint32_t hi = (uint32_t)(B >> 32), lo = (uint32_t)B;
+  if (((hi >> 20) & 0x7ffu) - 897u > 253u) return false;
+  uint32_t v = (((hi & 0x7fffffffu) - (896u << 20)) << 3) | (lo >> 29);
+  v += ((lo & 0x1fffffffu) + 0x0fffffffu + (v & 1u)) >> 29;
+  v |= hi & 0x80000000u;
+#ifdef __CUDA_ARCH__
+  *f = __int_as_float((int)v);
+#else
+  std::memcpy(f, &v, 4);
+#endif
+  return true;
+}
+
 } // namespace soft64
 
 #ifdef __CUDACC__
@@ -184,5 +222,17 @@ __device__ __forceinline__ double s64_fma_small(const soft64::Factor& f, double 
 __device__ __forceinline__ double s64_fma_small(double a, double b, double c)
 {
   return s64_fma_small(soft64::factor(a), a, b, c);
+}
+__device__ __forceinline__ double s64_from_float(float x)
+{
+  double d;
+  if (soft64::from_float(x, &d)) return d;
+  return (double)x;
+}
+__device__ __forceinline__ float s64_to_float(double x)
+{
+  float f;
+  if (soft64::to_float(x, &f)) return f;
+  return __double2float_rn(x);
 }
 #endif

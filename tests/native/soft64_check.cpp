@@ -46,11 +46,28 @@ int main(int argc, char** argv)
     check(1, soft64::mul(soft64::factor(a), b, &s), a * b);
     check(2, soft64::fma_small(soft64::factor(a), b, c, &s), std::fma(a, b, c));
   }
+  // conversions: every handled float exactly, doubles around the floats' ties and range ends
+  long conv = 0;
+  for (long i = 0; i < n; ++i)
+  {
+    const uint32_t u = (uint32_t)r();
+    float x, y;
+    std::memcpy(&x, &u, 4);
+    double s;
+    if (soft64::from_float(x, &s) && ++conv && soft64::bits(s) != soft64::bits((double)x)) ++wrong;
+    const uint64_t low[] = {0, 0x10000000u, 0x0fffffffu, 0x10000001u, r() & 0x1fffffffu};
+    const double d = make((r() & ~0x1fffffffULL) | low[i % 5], 890 + (int)(r() % 270));
+    const float want = (float)d;
+    if (soft64::to_float(d, &y) && ++conv && soft64::bits32(y) != soft64::bits32(want)) ++wrong;
+  }
+  if (conv < n) ++wrong; // most of them are handled
   // operands that no function may take: zeros, subnormals, infinities, NaN
   const double odd[] = {0.0, -0.0, 4.9e-324, -2.2e-308, INFINITY, -INFINITY, NAN};
   double s;
+  float g;
   for (double x : odd)
-    wrong += soft64::add(x, 1.0, &s) + soft64::add(1.0, x, &s) + soft64::add(x, x, &s) +
+    wrong += soft64::from_float((float)x, &s) + soft64::to_float(x, &g) + soft64::to_float(1e39, &g) +
+             soft64::to_float(1e-39, &g) + soft64::add(x, 1.0, &s) + soft64::add(1.0, x, &s) + soft64::add(x, x, &s) +
              soft64::mul(soft64::factor(x), 1.0, &s) + soft64::mul(soft64::factor(1.0), x, &s) +
              soft64::fma_small(soft64::factor(x), 1e-3, 1.0, &s) + soft64::fma_small(soft64::factor(1e-3), x, 1.0, &s) +
              soft64::fma_small(soft64::factor(1e-3), 1.0, x, &s);

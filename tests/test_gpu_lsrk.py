@@ -512,10 +512,11 @@ def test_evolve_rejects_bad_arguments(ctx, stslib):
 
 @pytest.mark.parametrize("nx,ny", [(390, 398), (391, 401), (683, 683), (1247, 1250), (1248, 1249)])
 @pytest.mark.parametrize("kind", [0, 1])
-def test_fp64_stage_rows_per_thread_bitwise(ctx, stslib, oracle, nx, ny, kind):
-    """The FP64 stage on both sides of the sizes where its rows per thread change (1, 2, 4 and 8
-    rows: 1, 3 and 10 times 1024 points per SM), with ragged last rows, forced and unforced: one
-    fixed step, bit for bit."""
+@pytest.mark.parametrize("mixed", [False, True])
+def test_rows_per_thread_bitwise(ctx, stslib, oracle, nx, ny, kind, mixed):
+    """The FP64 stage and the step end on both sides of the sizes where their rows per thread change
+    (1, 2, 4, then 8 or 16 rows: 1, 3 and 10 times 1024 points per SM), with ragged last rows and
+    columns, forced and unforced: one fixed step, bit for bit."""
     P = stslib.Problem(ctx, kind, nx, ny, 1.0, 0.3)
     O = oracle.Problem(kind, nx, ny, 1.0, 0.3)
     if kind:
@@ -524,8 +525,8 @@ def test_fp64_stage_rows_per_thread_bitwise(ctx, stslib, oracle, nx, ny, kind):
     else:
         y0, yo = P.initial(), O.initial()
     h = 30.0 / (8.0 * max(nx * nx, ny * ny))
-    I = stslib.LSRKStep(ctx, P, 0.0, y0, method=1, rtol=1e-6, atol=1e-10, hfixed=h)
-    J = oracle.Integrator(O, yo, method=1, rtol=1e-6, atol=1e-10, hfixed=h)
+    I = stslib.LSRKStep(ctx, P, 0.0, y0, method=1, rtol=1e-6, atol=1e-10, hfixed=h, mixed=mixed)
+    J = oracle.Integrator(O, yo, method=1, rtol=1e-6, atol=1e-10, hfixed=h, mixed=mixed)
     y = P.vector()
     I.evolve(h, y)
     assert J.evolve(h) == 0
