@@ -30,17 +30,22 @@ __device__ __forceinline__ void krylov_block_finish(xsum::Limbs* a, unsigned* fl
   t = __shfl_sync(0xffffffffu, t, 0);
   if (t != gridDim.x * gridDim.y - 1) return;
   __threadfence();
+  unsigned f[NACC];
 #pragma unroll
   for (int c = 0; c < NACC; ++c)
+  {
+    f[c] = 0;
     if (tid < xsum::NL) sm[c][0][tid] = (long long)atomicExch(&s->limbs[c][tid], 0ULL);
-  __syncwarp();
+    else if (tid == xsum::NL) f[c] = atomicExch(&s->flags[c], 0u);
+  }
+  if (tid == xsum::NL + 1) s->ticket = 0u;
+#pragma unroll
+  for (int c = 0; c < NACC; ++c) f[c] = __shfl_sync(0xffffffffu, f[c], xsum::NL);
   if (tid == 0)
   {
     double r[NACC];
 #pragma unroll
-    for (int c = 0; c < NACC; ++c) r[c] = xsum::finalize(sm[c][0], atomicExch(&s->flags[c], 0u));
+    for (int c = 0; c < NACC; ++c) r[c] = xsum::finalize(sm[c][0], f[c]);
     fin(r);
-    s->ticket = 0u;
-    __threadfence();
   }
 }

@@ -1083,7 +1083,7 @@ double sts_wrms_ewt(STS_Context ctx, const double* a, const double* b, const dou
                     double atol, int slot)
 {
   ctx_activate(ctx);
-  const int g = ew_blocks(ctx, n, 256 * 4);
+  const int g = red_blocks(ctx, n);
   if (b) wrms_ewt_kernel<1><<<g, 256, 0, ctx->stream>>>(n, a, b, y, rtol, atol, ctx->d_work, ctx->d_slots + slot);
   else wrms_ewt_kernel<0><<<g, 256, 0, ctx->stream>>>(n, a, b, y, rtol, atol, ctx->d_work, ctx->d_slots + slot);
   if (!STS_CUDA_OK(cudaStreamSynchronize(ctx->stream))) return NAN;
@@ -1631,7 +1631,7 @@ static int evolve_generic(LSRKMem* m, double tout, double clip, int itask)
       if (pf)
       {
         STS_Context ctx = m->ctx;
-        periodic_err_kernel<<<ew_blocks(ctx, m->n, 256 * 4), 256, 0, ctx->stream>>>(
+        periodic_err_kernel<<<red_blocks(ctx, m->n), 256, 0, ctx->stream>>>(
             m->n, NVD(y), NVD(yj), NVD(F), NVD(m->g_Fnew), 0.4 * h, m->rtol, m->atol, ctx->d_work,
             ctx->d_slots + SLOT_GENERIC);
         if (!STS_CUDA_OK(cudaStreamSynchronize(ctx->stream))) return STS_ERR_FAILURE;

@@ -188,24 +188,17 @@ __global__ void __launch_bounds__(256) maxnorm_kernel(long long n, const double*
     unsigned long long o = __shfl_xor_sync(0xffffffffu, m, s);
     m                    = o > m ? o : m;
   }
-  __shared__ bool last;
   if ((threadIdx.x & 31) == 0 && m) atomicMax(&w->maxbits, m);
   __syncthreads();
   if (threadIdx.x == 0)
   {
     __threadfence();
-    unsigned t = atomicAdd(&w->ticket, 1u);
-    last       = (t == gridDim.x - 1);
-  }
-  __syncthreads();
-  if (last && threadIdx.x == 0)
-  {
-    __threadfence();
-    unsigned long long b = atomicMax(&w->maxbits, 0ULL);
-    *slot                = __longlong_as_double((long long)b);
-    w->maxbits           = 0ULL;
-    w->ticket            = 0u;
-    __threadfence();
+    if (atomicAdd(&w->ticket, 1u) == gridDim.x - 1)
+    {
+      __threadfence();
+      *slot     = __longlong_as_double((long long)atomicExch(&w->maxbits, 0ULL));
+      w->ticket = 0u;
+    }
   }
 }
 
@@ -230,7 +223,7 @@ static double read_slot(STS_Context ctx, int slot)
 double sts_dot_exact(STS_Context ctx, const double* x, const double* y, long long n, int slot)
 {
   ctx_activate(ctx);
-  xred_kernel<0><<<ew_blocks(ctx, n, 256 * 4), 256, 0, ctx->stream>>>(n, x, y, ctx->d_work,
+  xred_kernel<0><<<red_blocks(ctx, n), 256, 0, ctx->stream>>>(n, x, y, ctx->d_work,
                                                                        ctx->d_slots + slot);
   return read_slot(ctx, slot);
 }
@@ -441,7 +434,7 @@ extern "C" double N_VWrmsNorm_Sts(N_Vector x, N_Vector w)
   STS_Context ctx = x->sunctx;
   long long n     = NVL(x);
   ctx_activate(ctx);
-  xred_kernel<1><<<ew_blocks(ctx, n, 256 * 4), 256, 0, ctx->stream>>>(n, NVD(x), NVD(w), ctx->d_work,
+  xred_kernel<1><<<red_blocks(ctx, n), 256, 0, ctx->stream>>>(n, NVD(x), NVD(w), ctx->d_work,
                                                                        ctx->d_slots + SLOT_GENERIC);
   return read_slot(ctx, SLOT_GENERIC);
 }
@@ -451,7 +444,7 @@ extern "C" double N_VMaxNorm_Sts(N_Vector x)
   STS_Context ctx = x->sunctx;
   long long n     = NVL(x);
   ctx_activate(ctx);
-  maxnorm_kernel<<<ew_blocks(ctx, n, 256 * 4), 256, 0, ctx->stream>>>(n, NVD(x), ctx->d_work,
+  maxnorm_kernel<<<red_blocks(ctx, n), 256, 0, ctx->stream>>>(n, NVD(x), ctx->d_work,
                                                                        ctx->d_slots + SLOT_GENERIC);
   return read_slot(ctx, SLOT_GENERIC);
 }
@@ -471,7 +464,7 @@ extern "C" int N_VDotProdMulti_Sts(int nvec, N_Vector x, N_Vector* Y, double* do
     for (int k = 0; k < cnt; ++k)
     {
       if (NVL(Y[c0 + k]) != n) return -1;
-      xred_kernel<0><<<ew_blocks(ctx, n, 256 * 4), 256, 0, ctx->stream>>>(n, NVD(x), NVD(Y[c0 + k]), ctx->d_work,
+      xred_kernel<0><<<red_blocks(ctx, n), 256, 0, ctx->stream>>>(n, NVD(x), NVD(Y[c0 + k]), ctx->d_work,
                                                                            ctx->d_slots + SLOT_MULTI + k);
     }
     if (!STS_CUDA_OK(cudaStreamSynchronize(ctx->stream))) return -1;

@@ -293,7 +293,7 @@ int sts_pcg_run(STS_Problem p, double gamma, N_Vector b, N_Vector x, double tol,
   hs.tolb = tol * bnorm;
   memset(w->h_out, 0, sizeof(PcgOut));
   cudaMemcpyAsync(w->d_s, &hs, sizeof(PcgScal), cudaMemcpyHostToDevice, st);
-  pcg_init_kernel<<<ew_blocks(ctx, n, 256 * 2), 256, 0, st>>>(n, NVD(b), w->d_s);
+  pcg_init_kernel<<<red_blocks(ctx, n), 256, 0, st>>>(n, NVD(b), w->d_s);
   // the graph is recorded for this x buffer
   cudaGraph_t g;
   if (!STS_CUDA_OK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal)))
