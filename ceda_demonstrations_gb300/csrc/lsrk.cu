@@ -1084,10 +1084,11 @@ double sts_wrms_ewt(STS_Context ctx, const double* a, const double* b, const dou
 {
   ctx_activate(ctx);
   const int g = red_blocks(ctx, n);
+  slot_arm(ctx, slot);
   if (b) wrms_ewt_kernel<1><<<g, 256, 0, ctx->stream>>>(n, a, b, y, rtol, atol, ctx->d_work, ctx->d_slots + slot);
   else wrms_ewt_kernel<0><<<g, 256, 0, ctx->stream>>>(n, a, b, y, rtol, atol, ctx->d_work, ctx->d_slots + slot);
-  if (!STS_CUDA_OK(cudaStreamSynchronize(ctx->stream))) return NAN;
-  return ((volatile double*)ctx->h_slots)[slot];
+  double v;
+  return slot_wait(ctx, slot, &v) ? v : NAN;
 }
 
 // controller update after an accepted step of size h with error dsm
@@ -1215,16 +1216,17 @@ static int evolve_fused(LSRKMem* m, double tout, double clip, int itask)
       STS_LSRKStageCoeffs(m->method, s, mu.data(), nu.data(), mus.data(), ajm1.data(), cjm1.data());
       m->nst_att++;
       fill_params(m, p, m->t, h, s, mu, nu, mus, ajm1, cjm1);
+      slot_arm(m->ctx, SLOT_DSM);
       if (run_step_fused(m, p, s)) return STS_ERR_FAILURE;
       m->interp_ready = false; // the attempt wrote y_{n+1} over the other parity buffer
-      if (!STS_CUDA_OK(cudaStreamSynchronize(st))) return STS_ERR_FAILURE;
+      double dsm;
+      if (!slot_wait(m->ctx, SLOT_DSM, &dsm)) return STS_ERR_FAILURE;
       if (const int ew = *(volatile int*)m->ctx->h_err)
       {
         *m->ctx->h_err = 0;
         sts_set_error("LSRKStep: %s in a stage kernel", sts_err_word_text(ew));
         return STS_ERR_FAILURE;
       }
-      const double dsm = ((volatile double*)m->ctx->h_slots)[SLOT_DSM];
       m->nfe += s;
       m->stages_total += s;
       if (s > m->stage_max) m->stage_max = s;
@@ -1631,11 +1633,11 @@ static int evolve_generic(LSRKMem* m, double tout, double clip, int itask)
       if (pf)
       {
         STS_Context ctx = m->ctx;
+        slot_arm(ctx, SLOT_GENERIC);
         periodic_err_kernel<<<red_blocks(ctx, m->n), 256, 0, ctx->stream>>>(
             m->n, NVD(y), NVD(yj), NVD(F), NVD(m->g_Fnew), 0.4 * h, m->rtol, m->atol, ctx->d_work,
             ctx->d_slots + SLOT_GENERIC);
-        if (!STS_CUDA_OK(cudaStreamSynchronize(ctx->stream))) return STS_ERR_FAILURE;
-        dsm = ((volatile double*)ctx->h_slots)[SLOT_GENERIC];
+        if (!slot_wait(ctx, SLOT_GENERIC, &dsm)) return STS_ERR_FAILURE;
       }
       else
       {

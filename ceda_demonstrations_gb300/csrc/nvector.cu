@@ -216,13 +216,14 @@ static void ew_launch(STS_Context ctx, long long n, double a, double b, const do
 
 static double read_slot(STS_Context ctx, int slot)
 {
-  if (!STS_CUDA_OK(cudaStreamSynchronize(ctx->stream))) return NAN;
-  return ((volatile double*)ctx->h_slots)[slot];
+  double v;
+  return slot_wait(ctx, slot, &v) ? v : NAN;
 }
 
 double sts_dot_exact(STS_Context ctx, const double* x, const double* y, long long n, int slot)
 {
   ctx_activate(ctx);
+  slot_arm(ctx, slot);
   xred_kernel<0><<<red_blocks(ctx, n), 256, 0, ctx->stream>>>(n, x, y, ctx->d_work,
                                                                        ctx->d_slots + slot);
   return read_slot(ctx, slot);
@@ -434,6 +435,7 @@ extern "C" double N_VWrmsNorm_Sts(N_Vector x, N_Vector w)
   STS_Context ctx = x->sunctx;
   long long n     = NVL(x);
   ctx_activate(ctx);
+  slot_arm(ctx, SLOT_GENERIC);
   xred_kernel<1><<<red_blocks(ctx, n), 256, 0, ctx->stream>>>(n, NVD(x), NVD(w), ctx->d_work,
                                                                        ctx->d_slots + SLOT_GENERIC);
   return read_slot(ctx, SLOT_GENERIC);
@@ -444,13 +446,14 @@ extern "C" double N_VMaxNorm_Sts(N_Vector x)
   STS_Context ctx = x->sunctx;
   long long n     = NVL(x);
   ctx_activate(ctx);
+  slot_arm(ctx, SLOT_GENERIC);
   maxnorm_kernel<<<red_blocks(ctx, n), 256, 0, ctx->stream>>>(n, NVD(x), ctx->d_work,
                                                                        ctx->d_slots + SLOT_GENERIC);
   return read_slot(ctx, SLOT_GENERIC);
 }
 
 // N_VDotProdMulti: the exact dot products of x with Y[0..nvec-1], each written to its own
-// result slot; one stream synchronisation per STS_NSLOTS - SLOT_MULTI products
+// result slot, waited for once per STS_NSLOTS - SLOT_MULTI products
 extern "C" int N_VDotProdMulti_Sts(int nvec, N_Vector x, N_Vector* Y, double* dots)
 {
   if (nvec < 1 || !x || !Y || !dots) return -1;
@@ -464,11 +467,12 @@ extern "C" int N_VDotProdMulti_Sts(int nvec, N_Vector x, N_Vector* Y, double* do
     for (int k = 0; k < cnt; ++k)
     {
       if (NVL(Y[c0 + k]) != n) return -1;
+      slot_arm(ctx, SLOT_MULTI + k);
       xred_kernel<0><<<red_blocks(ctx, n), 256, 0, ctx->stream>>>(n, NVD(x), NVD(Y[c0 + k]), ctx->d_work,
                                                                            ctx->d_slots + SLOT_MULTI + k);
     }
-    if (!STS_CUDA_OK(cudaStreamSynchronize(ctx->stream))) return -1;
-    for (int k = 0; k < cnt; ++k) dots[c0 + k] = ((volatile double*)ctx->h_slots)[SLOT_MULTI + k];
+    for (int k = 0; k < cnt; ++k)
+      if (!slot_wait(ctx, SLOT_MULTI + k, &dots[c0 + k])) return -1;
   }
   return 0;
 }

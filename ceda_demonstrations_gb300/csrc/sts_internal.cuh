@@ -81,6 +81,26 @@ struct STS_Context_ {
 
 bool ctx_activate(STS_Context ctx);
 
+// Results that the host waits for: it writes a bit pattern that no reduction produces into the
+// mapped slot before the launch and polls the slot, for some 0.2 ms, then falls back to the
+// stream's synchronisation (long kernels, errors, a value that happens to be the pattern). The
+// result is there 3-4 us before cudaStreamSynchronize returns. Kernels before it on the stream
+// have completed when it arrives.
+constexpr unsigned long long STS_SLOT_ARMED = 0x7ff4a5a5a5a5a5a5ULL;
+inline void slot_arm(STS_Context ctx, int slot)
+{
+  __atomic_store_n(reinterpret_cast<unsigned long long*>(ctx->h_slots) + slot, STS_SLOT_ARMED, __ATOMIC_RELEASE);
+}
+inline bool slot_wait(STS_Context ctx, int slot, double* value)
+{
+  const unsigned long long* p = reinterpret_cast<unsigned long long*>(ctx->h_slots) + slot;
+  bool ok                     = false;
+  for (int k = 0; k < 20000 && !ok; ++k) ok = __atomic_load_n(p, __ATOMIC_ACQUIRE) != STS_SLOT_ARMED;
+  if (!ok) ok = STS_CUDA_OK(cudaStreamSynchronize(ctx->stream));
+  *value = ((volatile double*)ctx->h_slots)[slot];
+  return ok;
+}
+
 // grid size for grid-stride elementwise / reduction kernels
 inline int ew_blocks(STS_Context ctx, long long n, int per_block)
 {
