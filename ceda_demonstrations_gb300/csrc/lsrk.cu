@@ -1351,47 +1351,120 @@ static int ssp_attempt(LSRKMem* m, double h, N_Vector y, N_Vector F, N_Vector yo
 // and the exact WRMS into one pass. Bit for bit the unfused sequence, with 40 instead of 64
 // bytes per point and stage and one kernel instead of seven per step end.
 // ---------------------------------------------------------------------------------------
+// Bound by the FP64 pipe, 17 instructions per point and stage in the reference's operation order;
+// the six products and the sums of face coefficients are integer code (soft64.cuh), eight
+// instructions are left. A thread marches down RY rows of its column (launch_stage64's rule), the
+// column's coefficients taken apart once. MEASURED_PERIODIC
+struct PeriodicColumn {
+  double w, e, sum;
+  soft64::Factor wF, eF;
+};
+
+__device__ __forceinline__ PeriodicColumn periodic_column(const ProbDev& P, long long i)
+{
+  PeriodicColumn c;
+  c.w   = P.Dxw[i];
+  c.e   = P.Dxe[i];
+  c.sum = c.w + c.e;
+  c.wF  = soft64::factor(c.w);
+  c.eF  = soft64::factor(c.e);
+  return c;
+}
+
+// periodic_point's operations on values at hand
+__device__ __forceinline__ double periodic_value(const PeriodicColumn& c, double s, double n, double uC, double uW,
+                                                 double uE, double uS, double uN)
+{
+  double v = s64_mul(-s64_add(c.sum, s64_add(s, n)), uC);
+  v        = __dadd_rn(v, s64_mul(c.wF, c.w, uW));
+  v        = __dadd_rn(v, s64_mul(c.eF, c.e, uE));
+  v        = __dadd_rn(v, s64_mul(s, uS));
+  v        = __dadd_rn(v, s64_mul(n, uN));
+  return v;
+}
+
+// f(i, j, k, value of the operator on u) for the rows of this thread
+template <int RY, typename F>
+__device__ __forceinline__ void periodic_march(const ProbDev& P, const double* __restrict__ u, F f)
+{
+  const long long nx = P.nx, ny = P.ny;
+  const long long i  = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const long long jb = ((long long)blockIdx.y * blockDim.y + threadIdx.y) * RY;
+  if (i >= nx || jb >= ny) return;
+  const long long je = jb + RY < ny ? jb + RY : ny;
+  const long long iw = (i == 0) ? nx - 1 : i - 1, ie = (i == nx - 1) ? 0 : i + 1;
+  const PeriodicColumn c = periodic_column(P, i);
+  double up = u[(jb == 0 ? ny - 1 : jb - 1) * nx + i], cur = u[jb * nx + i];
+#pragma unroll 1
+  for (long long j = jb; j < je; ++j)
+  {
+    const double dn = u[(j == ny - 1 ? 0 : j + 1) * nx + i];
+    const long long k = j * nx + i;
+    f(k, cur, periodic_value(c, __ldg(P.Dys + j), __ldg(P.Dyn + j), cur, u[j * nx + iw], u[j * nx + ie], up, dn));
+    up  = cur;
+    cur = dn;
+  }
+}
+
+template <int RY>
 __global__ void __launch_bounds__(256) periodic_stage_kernel(ProbDev P, double c0, double c1, double c2, double c3,
                                                              double c4, const double* __restrict__ ym1,
                                                              const double* __restrict__ ym2,
                                                              const double* __restrict__ y0,
                                                              const double* __restrict__ f0, double* __restrict__ yj)
 {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long j = (long long)blockIdx.y * blockDim.y + threadIdx.y;
-  if (i >= P.nx || j >= P.ny) return;
-  const long long k = j * P.nx + i;
-  const double fj   = periodic_point(P, ym1, i, j);
-  double acc        = __dmul_rn(c0, ym1[k]);
-  acc               = __fma_rn(c1, ym2[k], acc);
-  acc               = __fma_rn(c2, y0[k], acc);
-  acc               = __fma_rn(c3, fj, acc);
-  acc               = __fma_rn(c4, f0[k], acc);
-  yj[k]             = acc;
+  const soft64::Factor c0F = soft64::factor(c0);
+  periodic_march<RY>(P, ym1, [&](long long k, double u, double fj) {
+    double acc = s64_mul(c0F, c0, u);
+    acc        = __fma_rn(c1, ym2[k], acc);
+    acc        = __fma_rn(c2, y0[k], acc);
+    acc        = __fma_rn(c3, fj, acc);
+    acc        = __fma_rn(c4, f0[k], acc);
+    yj[k]      = acc;
+  });
 }
 
-__global__ void __launch_bounds__(256) periodic_err_kernel(long long n, const double* __restrict__ y,
+// step end: F(y_{n+1}) of ys, the error combination and its exact WRMS in one pass
+template <int RY>
+__global__ void __launch_bounds__(256) periodic_end_kernel(ProbDev P, const double* __restrict__ y,
                                                            const double* __restrict__ ys,
-                                                           const double* __restrict__ f0,
-                                                           const double* __restrict__ fs, double p4h, double rtol,
-                                                           double atol, RedWork* w, double* slot)
+                                                           const double* __restrict__ f0, double* __restrict__ fs,
+                                                           double p4h, double rtol, double atol, RedWork* w,
+                                                           double* slot)
 {
   xsum::Limbs acc;
   xsum::zero(acc);
-  unsigned flags         = 0;
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += stride)
-  {
+  unsigned flags = 0;
+  const soft64::Factor c8F = soft64::factor(0.8), rtF = soft64::factor(rtol);
+  periodic_march<RY>(P, ys, [&](long long k, double u, double f) {
+    fs[k]           = f;
     const double yv = y[k];
-    double e        = __dmul_rn(0.8, yv);
-    e               = __fma_rn(-0.8, ys[k], e);
+    double e        = s64_mul(c8F, 0.8, yv);
+    e               = __fma_rn(-0.8, u, e);
     e               = __fma_rn(p4h, f0[k], e);
-    e               = __fma_rn(p4h, fs[k], e);
-    const double wt = __drcp_rn(__dadd_rn(__dmul_rn(rtol, fabs(yv)), atol));
-    const double x  = __dmul_rn(e, wt);
-    xsum::add(acc, __dmul_rn(x, x), flags);
-  }
-  xsum_block_finish<256>(acc, flags, w, slot, 1, (double)n);
+    e               = __fma_rn(p4h, f, e);
+    const double wt = __drcp_rn(__dadd_rn(s64_mul(rtF, rtol, fabs(yv)), atol));
+    const double x  = s64_mul(e, wt);
+    xsum::add(acc, s64_mul(x, x), flags);
+  });
+  xsum_block_finish<256>(acc, flags, w, slot, 1, (double)(P.nx * P.ny));
+}
+
+// launch of a kernel that marches rows of a periodic problem: g(rows per thread, grid, block)
+template <typename G>
+static void periodic_rows(STS_Context ctx, STS_Problem p, G&& g)
+{
+  const long long n = p->nx * p->ny, W = 1024LL * ctx->num_sms;
+  const long long nyb = p->ny / (4 * 65535); // the grid's second dimension ends at 65535 blocks
+  auto go = [&](auto Rc) {
+    constexpr int R = decltype(Rc)::value;
+    const dim3 b(64, 4);
+    g(Rc, dim3((unsigned)((p->nx + b.x - 1) / b.x), (unsigned)((p->ny + b.y * R - 1) / (b.y * R))), b);
+  };
+  if (n < W && nyb < 1) go(std::integral_constant<int, 1>{});
+  else if (n < 3 * W && nyb < 2) go(std::integral_constant<int, 2>{});
+  else if (n < 10 * W && nyb < 4) go(std::integral_constant<int, 4>{});
+  else go(std::integral_constant<int, 8>{});
 }
 
 // Mixed reference mode: FP32 increments d_j = Y_j - Y_0 of the periodic problem in the
@@ -1603,9 +1676,10 @@ static int evolve_generic(LSRKMem* m, double tout, double clip, int itask)
         if (pf)
         {
           STS_Problem p = (STS_Problem)m->user_data;
-          const dim3 b(64, 4), g((unsigned)((p->nx + 63) / 64), (unsigned)((p->ny + 3) / 4));
-          periodic_stage_kernel<<<g, b, 0, m->ctx->stream>>>(p->dev, c[0], c[1], c[2], c[3], c[4], NVD(ym1),
-                                                             NVD(ym2), NVD(y), NVD(F), NVD(yj));
+          periodic_rows(m->ctx, p, [&](auto R, dim3 g, dim3 b) {
+            periodic_stage_kernel<decltype(R)::value><<<g, b, 0, m->ctx->stream>>>(
+              p->dev, c[0], c[1], c[2], c[3], c[4], NVD(ym1), NVD(ym2), NVD(y), NVD(F), NVD(yj));
+          });
         }
         else
         {
@@ -1617,7 +1691,7 @@ static int evolve_generic(LSRKMem* m, double tout, double clip, int itask)
         ym2 = ym1;
         ym1 = yj;
       }
-      if (frc == 0) frc = m->rhs(m->t + h, yj, m->g_Fnew, m->user_data);
+      if (frc == 0 && !pf) frc = m->rhs(m->t + h, yj, m->g_Fnew, m->user_data); // pf: in the step-end kernel
       m->nfe += s;
       if (frc < 0) return STS_RHSFUNC_FAIL;
       if (frc > 0)
@@ -1633,10 +1707,13 @@ static int evolve_generic(LSRKMem* m, double tout, double clip, int itask)
       if (pf)
       {
         STS_Context ctx = m->ctx;
+        STS_Problem p = (STS_Problem)m->user_data;
         slot_arm(ctx, SLOT_GENERIC);
-        periodic_err_kernel<<<red_blocks(ctx, m->n), 256, 0, ctx->stream>>>(
-            m->n, NVD(y), NVD(yj), NVD(F), NVD(m->g_Fnew), 0.4 * h, m->rtol, m->atol, ctx->d_work,
+        periodic_rows(ctx, p, [&](auto R, dim3 g, dim3 b) {
+          periodic_end_kernel<decltype(R)::value><<<g, b, 0, ctx->stream>>>(
+            p->dev, NVD(y), NVD(yj), NVD(F), NVD(m->g_Fnew), 0.4 * h, m->rtol, m->atol, ctx->d_work,
             ctx->d_slots + SLOT_GENERIC);
+        });
         if (!slot_wait(ctx, SLOT_GENERIC, &dsm)) return STS_ERR_FAILURE;
       }
       else
@@ -1655,9 +1732,18 @@ static int evolve_generic(LSRKMem* m, double tout, double clip, int itask)
       if (m->hfixed > 0.0 || dsm <= 1.0)
       {
         m->t = clipped ? clip : m->t + h;
-        cudaMemcpyAsync(NVD(m->g_yold), NVD(y), m->n * sizeof(double), cudaMemcpyDeviceToDevice, m->ctx->stream);
-        cudaMemcpyAsync(NVD(y), NVD(yj), m->n * sizeof(double), cudaMemcpyDeviceToDevice, m->ctx->stream);
-        cudaMemcpyAsync(NVD(F), NVD(m->g_Fnew), m->n * sizeof(double), cudaMemcpyDeviceToDevice, m->ctx->stream);
+        if (pf)
+        { // no user callback holds these buffers: y -> y_old, y_{n+1} -> y, F_{n+1} -> F by exchange
+          std::swap(NVC(m->g_yold)->data, NVC(y)->data);
+          std::swap(NVC(y)->data, NVC(yj)->data);
+          std::swap(NVC(F)->data, NVC(m->g_Fnew)->data);
+        }
+        else
+        {
+          cudaMemcpyAsync(NVD(m->g_yold), NVD(y), m->n * sizeof(double), cudaMemcpyDeviceToDevice, m->ctx->stream);
+          cudaMemcpyAsync(NVD(y), NVD(yj), m->n * sizeof(double), cudaMemcpyDeviceToDevice, m->ctx->stream);
+          cudaMemcpyAsync(NVD(F), NVD(m->g_Fnew), m->n * sizeof(double), cudaMemcpyDeviceToDevice, m->ctx->stream);
+        }
         accept_control(m, h, dsm);
         m->nst++;
         m->steps_since_dee++;
