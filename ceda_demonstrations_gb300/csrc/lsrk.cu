@@ -1353,8 +1353,9 @@ static int ssp_attempt(LSRKMem* m, double h, N_Vector y, N_Vector F, N_Vector yo
 // ---------------------------------------------------------------------------------------
 // Bound by the FP64 pipe, 17 instructions per point and stage in the reference's operation order;
 // the six products and the sums of face coefficients are integer code (soft64.cuh), eight
-// instructions are left. A thread marches down RY rows of its column (launch_stage64's rule), the
-// column's coefficients taken apart once. MEASURED_PERIODIC
+// instructions are left. A thread marches down RY rows of its column, the column's coefficients
+// taken apart once. Stage at 1000 x 768 29.4 -> 22.6 us, at 2048^2 97; the integer side and the FP64
+// pipe are then equally busy (a product more or less as integer code: 94 to 100 us).
 struct PeriodicColumn {
   double w, e, sum;
   soft64::Factor wF, eF;
@@ -1450,7 +1451,9 @@ __global__ void __launch_bounds__(256) periodic_end_kernel(ProbDev P, const doub
   xsum_block_finish<256>(acc, flags, w, slot, 1, (double)(P.nx * P.ny));
 }
 
-// launch of a kernel that marches rows of a periodic problem: g(rows per thread, grid, block)
+// launch of a kernel that marches rows of a periodic problem: g(rows per thread, grid, block).
+// Measured us per stage with 1 / 2 / 4 / 8 rows (W: the resident threads, 1024 per SM): 128^2 5.1 /
+// 6.1 / - / 14.4, 1000 x 768 (5 W) 22.7 / 22.6 / 24.6 / 24.7, 2048^2 (27 W) 104 / 96 / 97 / 97.
 template <typename G>
 static void periodic_rows(STS_Context ctx, STS_Problem p, G&& g)
 {
@@ -1462,8 +1465,7 @@ static void periodic_rows(STS_Context ctx, STS_Problem p, G&& g)
     g(Rc, dim3((unsigned)((p->nx + b.x - 1) / b.x), (unsigned)((p->ny + b.y * R - 1) / (b.y * R))), b);
   };
   if (n < W && nyb < 1) go(std::integral_constant<int, 1>{});
-  else if (n < 3 * W && nyb < 2) go(std::integral_constant<int, 2>{});
-  else if (n < 10 * W && nyb < 4) go(std::integral_constant<int, 4>{});
+  else if (n < 10 * W && nyb < 2) go(std::integral_constant<int, 2>{});
   else go(std::integral_constant<int, 8>{});
 }
 
