@@ -20,12 +20,14 @@
 //   definite operator, so it preconditions CG.
 // Every kernel is elementwise with an explicit operation order (fused multiply-adds written
 // out), so the CPU oracle reproduces the V-cycle bit for bit. The cycle for a given gamma is
-// captured once in a CUDA graph (about 7 kernels per level, ~22 levels at 2048^2).
+// captured once in a CUDA graph (10 kernels per level, 12 levels at 2048^2, one kernel for the rest).
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <vector>
 
+#include "kernels.cuh"
 #include "sts_internal.cuh"
 
 namespace {
@@ -33,6 +35,7 @@ namespace {
 constexpr double PFMG_OMEGA = 0.8; // weighted-Jacobi factor (2-D five-point stencil)
 constexpr int PFMG_COARSE_SWEEPS = 8;
 constexpr int PFMG_MAX_LEVELS    = 64;
+constexpr long long SOFT_POINTS  = 1 << 19; // levels from here on are bound by throughput
 
 struct PfmgLevel {
   long long nx = 0, ny = 0;
@@ -50,30 +53,68 @@ __device__ __forceinline__ double at(const double* u, long long nx, long long ny
   return (i >= 0 && i < nx && j >= 0 && j < ny) ? u[j * nx + i] : 0.0;
 }
 
+// Products and neighbour sums of M u as integer code (soft64.cuh) on large levels (SOFT), which the
+// FP64 pipe bounds, as FP64 instructions where latency does. V-cycle at 2048^2, red/black (Jacobi):
+// 812 (913) us without, 742 (847) with the products, 717 (763) with the sums too; 500 x 300 with
+// both from its size on 178 us, without 172. The Gauss-Seidel sums stay FP64: its passes are bound
+// by L2 traffic (735 and 738 us with either).
+template <bool SOFT>
+__device__ __forceinline__ double mul(double a, double b) { return SOFT ? s64_mul(a, b) : __dmul_rn(a, b); }
+template <bool SOFT>
+__device__ __forceinline__ double add(double a, double b) { return SOFT ? s64_add(a, b) : __dadd_rn(a, b); }
+
 // M u at (i, j): d u - a_x (u_w + u_e) - a_y (u_s + u_n)
+template <bool SOFT>
 __device__ __forceinline__ double apply_m(const double* u, long long nx, long long ny, long long i, long long j,
                                           double ax, double ay, double d)
 {
-  const double sx = at(u, nx, ny, i - 1, j) + at(u, nx, ny, i + 1, j);
-  const double sy = at(u, nx, ny, i, j - 1) + at(u, nx, ny, i, j + 1);
-  double m        = d * u[j * nx + i];
+  const double sx = add<SOFT>(at(u, nx, ny, i - 1, j), at(u, nx, ny, i + 1, j));
+  const double sy = add<SOFT>(at(u, nx, ny, i, j - 1), at(u, nx, ny, i, j + 1));
+  double m        = mul<SOFT>(d, u[j * nx + i]);
   m               = __fma_rn(-ax, sx, m);
   m               = __fma_rn(-ay, sy, m);
   return m;
 }
 
-// weighted Jacobi: out = in + wd (f - M in)
+// weighted Jacobi: in + wd (f - M in)
+template <bool SOFT>
+__device__ __forceinline__ double jacobi_point(const double* in, const double* f, long long nx, long long ny,
+                                               long long i, long long j, double ax, double ay, double d, double wd)
+{
+  const long long k = j * nx + i;
+  return __fma_rn(wd, f[k] - apply_m<SOFT>(in, nx, ny, i, j, ax, ay, d), in[k]);
+}
+
+template <bool SOFT>
 __global__ void jacobi_kernel(long long nx, long long ny, double ax, double ay, double d, double wd,
                               const double* __restrict__ f, const double* __restrict__ in, double* __restrict__ out)
 {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long j = (long long)blockIdx.y * blockDim.y + threadIdx.y;
   if (i >= nx || j >= ny) return;
-  const long long k = j * nx + i;
-  out[k]            = __fma_rn(wd, f[k] - apply_m(in, nx, ny, i, j, ax, ay, d), in[k]);
+  out[j * nx + i] = jacobi_point<SOFT>(in, f, nx, ny, i, j, ax, ay, d, wd);
 }
 
-// Gauss-Seidel on the points with (i + j) % 2 == color: u = dinv (f + a_x (u_w + u_e) + a_y (u_s + u_n))
+// Gauss-Seidel value dinv (f + a_x (u_w + u_e) + a_y (u_s + u_n))
+template <bool SOFT>
+__device__ __forceinline__ double gs_value(double f, double uw, double ue, double us, double un, double ax, double ay,
+                                           double dinv)
+{
+  double v = __fma_rn(ax, uw + ue, f);
+  v        = __fma_rn(ay, us + un, v);
+  return mul<SOFT>(dinv, v);
+}
+
+template <bool SOFT>
+__device__ __forceinline__ double gs_point(const double* u, const double* f, long long nx, long long ny, long long i,
+                                           long long j, double ax, double ay, double dinv)
+{
+  return gs_value<SOFT>(f[j * nx + i], at(u, nx, ny, i - 1, j), at(u, nx, ny, i + 1, j), at(u, nx, ny, i, j - 1),
+                  at(u, nx, ny, i, j + 1), ax, ay, dinv);
+}
+
+// the points with (i + j) % 2 == color
+template <bool SOFT>
 __global__ void rbgs_kernel(long long nx, long long ny, double ax, double ay, double dinv, const double* __restrict__ f,
                             double* u, int color)
 {
@@ -81,67 +122,96 @@ __global__ void rbgs_kernel(long long nx, long long ny, double ax, double ay, do
   const long long j = (long long)blockIdx.y * blockDim.y + threadIdx.y;
   const long long ii = i + ((j + color) & 1); // the point of this color in the pair (i, i+1)
   if (ii >= nx || j >= ny) return;
-  const double sx = at(u, nx, ny, ii - 1, j) + at(u, nx, ny, ii + 1, j);
-  const double sy = at(u, nx, ny, ii, j - 1) + at(u, nx, ny, ii, j + 1);
-  double v        = __fma_rn(ax, sx, f[j * nx + ii]);
-  v               = __fma_rn(ay, sy, v);
-  u[j * nx + ii]  = dinv * v;
+  u[j * nx + ii] = gs_point<SOFT>(u, f, nx, ny, ii, j, ax, ay, dinv);
 }
 
-__global__ void residual_kernel(long long nx, long long ny, double ax, double ay, double d, const double* __restrict__ f,
-                                const double* __restrict__ u, double* __restrict__ r)
+// the first half sweep from a zero guess: a red point is dinv f (-0 as the sum with zero gives it).
+// The black half sweep after it writes the black points without reading them, so the guess is
+// never stored. (Both colors in one pass, the red neighbours formed again: 76 us at 2048^2 against
+// 10 + 19.)
+template <bool SOFT>
+__global__ void red_first_kernel(long long nx, long long ny, double dinv, const double* __restrict__ f,
+                                 double* __restrict__ u)
 {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long j = (long long)blockIdx.y * blockDim.y + threadIdx.y;
+  const long long i = 2 * ((long long)blockIdx.x * blockDim.x + threadIdx.x) + (j & 1);
   if (i >= nx || j >= ny) return;
-  r[j * nx + i] = f[j * nx + i] - apply_m(u, nx, ny, i, j, ax, ay, d);
+  const double v = f[j * nx + i];
+  u[j * nx + i]  = mul<SOFT>(dinv, (__double_as_longlong(v) << 1) == 0 ? 0.0 : v);
 }
 
-// full weighting in direction dir onto the coarse grid (cnx x cny): fc = 0.5 b + 0.25 (a + c)
-__global__ void restrict_kernel(long long nx, long long ny, int dir, long long cnx, long long cny,
-                                const double* __restrict__ r, double* __restrict__ fc)
+// residual f - M u at (i, j), zero outside
+template <bool SOFT>
+__device__ __forceinline__ double residual_at(const double* f, const double* u, long long nx, long long ny, long long i,
+                                              long long j, double ax, double ay, double d)
 {
-  const long long I = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long J = (long long)blockIdx.y * blockDim.y + threadIdx.y;
-  if (I >= cnx || J >= cny) return;
-  double a, b, c;
+  return (i < nx && j < ny) ? f[j * nx + i] - apply_m<SOFT>(u, nx, ny, i, j, ax, ay, d) : 0.0;
+}
+
+// full weighting in direction dir onto the coarse grid (cnx x cny): fc = 0.5 b + 0.25 (a + c) of the
+// residuals at fine 2I, 2I+1, 2I+2, formed on the way. RC coarse rows per thread, so that c of
+// one is a of the next (dir 1); in a row c comes from the next lane (dir 0).
+template <int RC, bool SOFT>
+__global__ void residual_restrict_kernel(long long nx, long long ny, double ax, double ay, double d, int dir,
+                                         long long cnx, long long cny, const double* __restrict__ f,
+                                         const double* __restrict__ u, double* __restrict__ fc)
+{
+  const long long I  = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const long long J0 = ((long long)blockIdx.y * blockDim.y + threadIdx.y) * RC;
+  auto res = [&](long long i, long long j) { return residual_at<SOFT>(f, u, nx, ny, i, j, ax, ay, d); };
   if (dir == 0)
-  {
-    a = at(r, nx, ny, 2 * I, J);
-    b = at(r, nx, ny, 2 * I + 1, J);
-    c = at(r, nx, ny, 2 * I + 2, J);
+  { // (whole warps: 32 lanes of one row, shuffles before any exit)
+    for (long long J = J0; J < J0 + RC; ++J)
+    {
+      const double a = res(2 * I, J);
+      double c       = __shfl_down_sync(0xffffffffu, a, 1);
+      if (I >= cnx || J >= cny) continue;
+      if ((threadIdx.x & 31) == 31) c = res(2 * I + 2, J);
+      fc[J * cnx + I] = __fma_rn(0.5, res(2 * I + 1, J), 0.25 * (a + c));
+    }
+    return;
   }
-  else
+  if (I >= cnx || J0 >= cny) return;
+  double a = res(I, 2 * J0);
+  for (long long J = J0; J < J0 + RC && J < cny; ++J)
   {
-    a = at(r, nx, ny, I, 2 * J);
-    b = at(r, nx, ny, I, 2 * J + 1);
-    c = at(r, nx, ny, I, 2 * J + 2);
+    const double b = res(I, 2 * J + 1), c = res(I, 2 * J + 2);
+    fc[J * cnx + I] = __fma_rn(0.5, b, 0.25 * (a + c));
+    a               = c;
   }
-  fc[J * cnx + I] = __fma_rn(0.5, b, 0.25 * (a + c));
 }
 
-// u += P uc (linear interpolation in direction dir)
-__global__ void prolong_kernel(long long nx, long long ny, int dir, long long cnx, long long cny,
-                               const double* __restrict__ uc, double* __restrict__ u)
+// the same from stored residuals
+__device__ __forceinline__ double restrict_point(const double* r, long long nx, long long ny, int dir, long long I,
+                                                 long long J)
 {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const double a = dir == 0 ? at(r, nx, ny, 2 * I, J) : at(r, nx, ny, I, 2 * J);
+  const double b = dir == 0 ? at(r, nx, ny, 2 * I + 1, J) : at(r, nx, ny, I, 2 * J + 1);
+  const double c = dir == 0 ? at(r, nx, ny, 2 * I + 2, J) : at(r, nx, ny, I, 2 * J + 2);
+  return __fma_rn(0.5, b, 0.25 * (a + c));
+}
+
+// P uc at fine (i, j): linear interpolation in direction dir
+__device__ __forceinline__ double interpolate(const double* uc, long long i, long long j, int dir, long long cnx,
+                                              long long cny)
+{
+  const long long q = dir == 0 ? i : j, Q = q >> 1;
+  if (q & 1) return dir == 0 ? at(uc, cnx, cny, Q, j) : at(uc, cnx, cny, i, Q);
+  const double lo = dir == 0 ? at(uc, cnx, cny, Q - 1, j) : at(uc, cnx, cny, i, Q - 1); // between coarse Q - 1 and Q
+  const double hi = dir == 0 ? at(uc, cnx, cny, Q, j) : at(uc, cnx, cny, i, Q);
+  return 0.5 * (lo + hi);
+}
+
+// u += P uc: on every point (color -1), or on the points of one color, where the Gauss-Seidel half
+// sweep that follows overwrites the others without reading them
+__global__ void prolong_kernel(long long nx, long long ny, int dir, long long cnx, long long cny,
+                               const double* __restrict__ uc, double* __restrict__ u, int color)
+{
+  long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long j = (long long)blockIdx.y * blockDim.y + threadIdx.y;
+  if (color >= 0) i = 2 * i + ((j + color) & 1);
   if (i >= nx || j >= ny) return;
-  const long long q = dir == 0 ? i : j;
-  double e;
-  if (q & 1)
-  {
-    const long long Q = q >> 1;
-    e = dir == 0 ? at(uc, cnx, cny, Q, j) : at(uc, cnx, cny, i, Q);
-  }
-  else
-  {
-    const long long Q = q >> 1; // between coarse Q - 1 and Q
-    const double lo = dir == 0 ? at(uc, cnx, cny, Q - 1, j) : at(uc, cnx, cny, i, Q - 1);
-    const double hi = dir == 0 ? at(uc, cnx, cny, Q, j) : at(uc, cnx, cny, i, Q);
-    e = 0.5 * (lo + hi);
-  }
-  u[j * nx + i] += e;
+  u[j * nx + i] += interpolate(uc, i, j, dir, cnx, cny);
 }
 
 // ---- periodic levels (the reference's problem): variable face couplings, wrapped neighbours.
@@ -180,41 +250,76 @@ __device__ __forceinline__ double per_m(const PerPoint& q, double uc)
   return m;
 }
 
+__device__ __forceinline__ double per_jacobi_point(long long nx, long long ny, const double* axf, const double* ayf,
+                                                   const double* f, const double* in, long long i, long long j)
+{
+  const long long k = j * nx + i;
+  const PerPoint q  = per_point(in, nx, ny, i, j, axf, ayf);
+  const double wd   = PFMG_OMEGA * (1.0 / q.d);
+  return __fma_rn(wd, f[k] - per_m(q, in[k]), in[k]);
+}
+
+// one colour of red/black Gauss-Seidel from `in` (the other colour copied): on odd periodic
+// sizes, where two points of one colour meet across the wrap, the sweep stays deterministic
+__device__ __forceinline__ double per_rbgs_point(long long nx, long long ny, const double* axf, const double* ayf,
+                                                 const double* f, const double* in, long long i, long long j, int color)
+{
+  const long long k = j * nx + i;
+  if (((i + j) & 1) != color) return in[k];
+  const PerPoint q = per_point(in, nx, ny, i, j, axf, ayf);
+  double v         = __fma_rn(q.w, q.uW, f[k]);
+  v                = __fma_rn(q.e, q.uE, v);
+  v                = __fma_rn(q.s, q.uS, v);
+  v                = __fma_rn(q.n, q.uN, v);
+  return v / q.d;
+}
+
+__device__ __forceinline__ double per_residual_point(long long nx, long long ny, const double* axf, const double* ayf,
+                                                     const double* f, const double* u, long long i, long long j)
+{
+  const PerPoint q = per_point(u, nx, ny, i, j, axf, ayf);
+  return f[j * nx + i] - per_m(q, u[j * nx + i]);
+}
+
+// full weighting with wrap: coarse I <- fine 2I, 2I+1, 2I+2 (mod n)
+__device__ __forceinline__ double per_restrict_point(long long nx, long long ny, int dir, const double* r, long long I,
+                                                     long long J)
+{
+  const double a = dir == 0 ? r[J * nx + 2 * I] : r[(2 * J) * nx + I];
+  const double b = dir == 0 ? r[J * nx + 2 * I + 1] : r[(2 * J + 1) * nx + I];
+  const double c = dir == 0 ? r[J * nx + wrap(2 * I + 2, nx)] : r[wrap(2 * J + 2, ny) * nx + I];
+  return __fma_rn(0.5, b, 0.25 * (a + c));
+}
+
+// P uc with wrap: fine 2Q+1 <- coarse Q, fine 2Q <- mean of coarse Q-1 (mod) and Q
+__device__ __forceinline__ double per_interpolate(const double* uc, long long i, long long j, int dir, long long cnx,
+                                                  long long cny)
+{
+  const long long q = dir == 0 ? i : j;
+  const long long Q = q >> 1;
+  if (q & 1) return dir == 0 ? uc[j * cnx + Q] : uc[Q * cnx + i];
+  const long long Qm = wrap(Q - 1, dir == 0 ? cnx : cny);
+  const double lo    = dir == 0 ? uc[j * cnx + Qm] : uc[Qm * cnx + i];
+  const double hi    = dir == 0 ? uc[j * cnx + Q] : uc[Q * cnx + i];
+  return 0.5 * (lo + hi);
+}
+
 __global__ void per_jacobi_kernel(long long nx, long long ny, const double* __restrict__ axf,
                                   const double* __restrict__ ayf, const double* __restrict__ f,
                                   const double* __restrict__ in, double* __restrict__ out)
 {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long j = (long long)blockIdx.y * blockDim.y + threadIdx.y;
-  if (i >= nx || j >= ny) return;
-  const long long k = j * nx + i;
-  const PerPoint q  = per_point(in, nx, ny, i, j, axf, ayf);
-  const double wd   = PFMG_OMEGA * (1.0 / q.d);
-  out[k]            = __fma_rn(wd, f[k] - per_m(q, in[k]), in[k]);
+  if (i < nx && j < ny) out[j * nx + i] = per_jacobi_point(nx, ny, axf, ayf, f, in, i, j);
 }
 
-// one colour of red/black Gauss-Seidel from `in` into `out` (the other colour copied): on odd
-// periodic sizes, where two points of one colour meet across the wrap, the sweep stays
-// deterministic
 __global__ void per_rbgs_kernel(long long nx, long long ny, const double* __restrict__ axf,
                                 const double* __restrict__ ayf, const double* __restrict__ f,
                                 const double* __restrict__ in, double* __restrict__ out, int color)
 {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long j = (long long)blockIdx.y * blockDim.y + threadIdx.y;
-  if (i >= nx || j >= ny) return;
-  const long long k = j * nx + i;
-  if (((i + j) & 1) != color)
-  {
-    out[k] = in[k];
-    return;
-  }
-  const PerPoint q = per_point(in, nx, ny, i, j, axf, ayf);
-  double v         = __fma_rn(q.w, q.uW, f[k]);
-  v                = __fma_rn(q.e, q.uE, v);
-  v                = __fma_rn(q.s, q.uS, v);
-  v                = __fma_rn(q.n, q.uN, v);
-  out[k]           = v / q.d;
+  if (i < nx && j < ny) out[j * nx + i] = per_rbgs_point(nx, ny, axf, ayf, f, in, i, j, color);
 }
 
 __global__ void per_residual_kernel(long long nx, long long ny, const double* __restrict__ axf,
@@ -223,53 +328,117 @@ __global__ void per_residual_kernel(long long nx, long long ny, const double* __
 {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long j = (long long)blockIdx.y * blockDim.y + threadIdx.y;
-  if (i >= nx || j >= ny) return;
-  const PerPoint q = per_point(u, nx, ny, i, j, axf, ayf);
-  r[j * nx + i]    = f[j * nx + i] - per_m(q, u[j * nx + i]);
+  if (i < nx && j < ny) r[j * nx + i] = per_residual_point(nx, ny, axf, ayf, f, u, i, j);
 }
 
-// full weighting with wrap: coarse I <- fine 2I, 2I+1, 2I+2 (mod n)
 __global__ void per_restrict_kernel(long long nx, long long ny, int dir, long long cnx, long long cny,
                                     const double* __restrict__ r, double* __restrict__ fc)
 {
   const long long I = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long J = (long long)blockIdx.y * blockDim.y + threadIdx.y;
-  if (I >= cnx || J >= cny) return;
-  double a, b, c;
-  if (dir == 0)
-  {
-    a = r[J * nx + 2 * I];
-    b = r[J * nx + 2 * I + 1];
-    c = r[J * nx + wrap(2 * I + 2, nx)];
-  }
-  else
-  {
-    a = r[(2 * J) * nx + I];
-    b = r[(2 * J + 1) * nx + I];
-    c = r[wrap(2 * J + 2, ny) * nx + I];
-  }
-  fc[J * cnx + I] = __fma_rn(0.5, b, 0.25 * (a + c));
+  if (I < cnx && J < cny) fc[J * cnx + I] = per_restrict_point(nx, ny, dir, r, I, J);
 }
 
-// u += P uc with wrap: fine 2Q+1 <- coarse Q, fine 2Q <- mean of coarse Q-1 (mod) and Q
 __global__ void per_prolong_kernel(long long nx, long long ny, int dir, long long cnx, long long cny,
                                    const double* __restrict__ uc, double* __restrict__ u)
 {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long j = (long long)blockIdx.y * blockDim.y + threadIdx.y;
-  if (i >= nx || j >= ny) return;
-  const long long q = dir == 0 ? i : j;
-  const long long Q = q >> 1;
-  double e;
-  if (q & 1) e = dir == 0 ? uc[j * cnx + Q] : uc[Q * cnx + i];
-  else
+  if (i < nx && j < ny) u[j * nx + i] += per_interpolate(uc, i, j, dir, cnx, cny);
+}
+
+// ---- the coarse end of the cycle in one block
+// On small levels the launches (2 us each) cost more than the arithmetic, so one block runs all the
+// levels up to 1024 points, a point per thread, the fields in L1 / L2, a block barrier between
+// sweeps. The point operations are those of the kernels above. V-cycle at 128^2 146 us, at 2048^2
+// 717 (every level launched, fields zeroed, residuals stored: 1003).
+constexpr long long BOTTOM_POINTS = 1024; // a point per thread
+constexpr int BOTTOM_LEVELS       = 24;
+
+struct BottomLevel {
+  int nx, ny, dir;
+  double ax, ay, d, dinv, wd;
+  double *f, *u, *t;
+  const double *axf, *ayf;
+};
+
+struct BottomArgs {
+  int nl, relax, nrelax;
+  BottomLevel l[BOTTOM_LEVELS];
+};
+
+template <bool PERIODIC>
+__device__ __forceinline__ void bottom_smooth(const BottomLevel& l, int relax, int sweeps, bool post, int i, int j)
+{
+  const bool own = j < l.ny; // this thread's point (i, j)
+  const int k    = j * l.nx + i;
+  double *in = l.u, *out = l.t;
+  for (int s = 0; s < sweeps; ++s)
   {
-    const long long Qm = wrap(Q - 1, dir == 0 ? cnx : cny);
-    const double lo    = dir == 0 ? uc[j * cnx + Qm] : uc[Qm * cnx + i];
-    const double hi    = dir == 0 ? uc[j * cnx + Q] : uc[Q * cnx + i];
-    e                  = 0.5 * (lo + hi);
+    if (relax == 1)
+    {
+      if (own)
+        out[k] = PERIODIC ? per_jacobi_point(l.nx, l.ny, l.axf, l.ayf, l.f, in, i, j)
+                          : jacobi_point<false>(in, l.f, l.nx, l.ny, i, j, l.ax, l.ay, l.d, l.wd);
+      __syncthreads();
+      double* q = in;
+      in        = out;
+      out       = q;
+      continue;
+    }
+    for (int h = 0; h < 2; ++h)
+    {
+      const int color = (post && relax == 2) ? 1 - h : h;
+      if (PERIODIC)
+      {
+        if (own) out[k] = per_rbgs_point(l.nx, l.ny, l.axf, l.ayf, l.f, in, i, j, color);
+        double* q = in;
+        in        = out;
+        out       = q;
+      }
+      else if (own && ((i + j) & 1) == color) l.u[k] = gs_point<false>(l.u, l.f, l.nx, l.ny, i, j, l.ax, l.ay, l.dinv);
+      __syncthreads();
+    }
   }
-  u[j * nx + i] += e;
+  if (in != l.u)
+  {
+    if (own) l.u[k] = in[k];
+    __syncthreads();
+  }
+}
+
+template <bool PERIODIC>
+__global__ void __launch_bounds__(BOTTOM_POINTS) bottom_kernel(const __grid_constant__ BottomArgs B)
+{
+  const int k = threadIdx.x;
+  for (int v = 0; v < B.nl; ++v)
+  {
+    const BottomLevel& l = B.l[v];
+    const int i = k % l.nx, j = k / l.nx;
+    if (j < l.ny) l.u[k] = 0.0;
+    __syncthreads();
+    bottom_smooth<PERIODIC>(l, B.relax, l.dir < 0 ? PFMG_COARSE_SWEEPS : B.nrelax, false, i, j);
+    if (l.dir < 0) break;
+    const BottomLevel& c = B.l[v + 1];
+    if (j < l.ny)
+      l.t[k] = PERIODIC ? per_residual_point(l.nx, l.ny, l.axf, l.ayf, l.f, l.u, i, j)
+                        : residual_at<false>(l.f, l.u, l.nx, l.ny, i, j, l.ax, l.ay, l.d);
+    __syncthreads();
+    if (k < c.nx * c.ny)
+      c.f[k] = PERIODIC ? per_restrict_point(l.nx, l.ny, l.dir, l.t, k % c.nx, k / c.nx)
+                        : restrict_point(l.t, l.nx, l.ny, l.dir, k % c.nx, k / c.nx);
+    __syncthreads();
+  }
+  for (int v = B.nl - 2; v >= 0; --v)
+  {
+    const BottomLevel& l = B.l[v];
+    const BottomLevel& c = B.l[v + 1];
+    const int i = k % l.nx, j = k / l.nx;
+    if (j < l.ny)
+      l.u[k] += PERIODIC ? per_interpolate(c.u, i, j, l.dir, c.nx, c.ny) : interpolate(c.u, i, j, l.dir, c.nx, c.ny);
+    __syncthreads();
+    bottom_smooth<PERIODIC>(l, B.relax, B.nrelax, true, i, j);
+  }
 }
 
 dim3 blocks2d(long long nx, long long ny, dim3 b) { return dim3((unsigned)((nx + b.x - 1) / b.x), (unsigned)((ny + b.y - 1) / b.y)); }
@@ -294,23 +463,47 @@ struct STS_PFMG_ {
   std::vector<double> dxe, dyn; // periodic problems: the problem's face coefficients (host copy)
   double gamma    = NAN; // the gamma the hierarchy and graph were built for
   std::vector<PfmgLevel> L;
+  double* arena         = nullptr; // the device fields of all levels, one allocation
   cudaGraphExec_t graph = nullptr;
   long long vcycles = 0;
 };
 
 static void pfmg_free_levels(STS_PFMG mg)
 {
-  for (auto& l : mg->L)
-  {
-    cudaFree(l.f);
-    cudaFree(l.u);
-    cudaFree(l.t);
-    if (l.axf) cudaFree(l.axf);
-    if (l.ayf) cudaFree(l.ayf);
-  }
+  cudaFree(mg->arena);
+  mg->arena = nullptr;
   mg->L.clear();
   if (mg->graph) cudaGraphExecDestroy(mg->graph);
   mg->graph = nullptr;
+}
+
+// fields of every level from one allocation (a hierarchy at 2048^2 has 63 of them; as many
+// cudaMalloc and cudaFree calls took a millisecond and more per setup)
+static bool pfmg_alloc(STS_PFMG mg)
+{
+  auto up    = [](long long n) { return (n + 31) / 32 * 32; };
+  long long total = 0;
+  for (const PfmgLevel& l : mg->L) total += 3 * up(l.nx * l.ny) + (mg->periodic ? up(l.nx) + up(l.ny) : 0);
+  if (!STS_CUDA_OK(cudaMalloc(&mg->arena, (size_t)total * sizeof(double)))) return false;
+  double* q = mg->arena;
+  auto take = [&](long long n) {
+    double* r = q;
+    q += up(n);
+    return r;
+  };
+  for (PfmgLevel& l : mg->L)
+  {
+    l.f = take(l.nx * l.ny);
+    l.u = take(l.nx * l.ny);
+    l.t = take(l.nx * l.ny);
+    if (!mg->periodic) continue;
+    l.axf = take(l.nx);
+    l.ayf = take(l.ny);
+    if (!STS_CUDA_OK(cudaMemcpy(l.axf, l.hax.data(), l.nx * sizeof(double), cudaMemcpyHostToDevice)) ||
+        !STS_CUDA_OK(cudaMemcpy(l.ayf, l.hay.data(), l.ny * sizeof(double), cudaMemcpyHostToDevice)))
+      return false;
+  }
+  return true;
 }
 
 // the level hierarchy of M = I - gamma A (host rules, restated in the oracle)
@@ -355,20 +548,10 @@ static bool pfmg_build_periodic(STS_PFMG mg, double gamma)
     if (cx && (axm >= aym || !cy)) l.dir = 0;
     else if (cy) l.dir = 1;
     else l.dir = -1;
-    const size_t bytes = (size_t)(l.nx * l.ny) * sizeof(double);
-    if (!STS_CUDA_OK(cudaMalloc(&l.f, bytes)) || !STS_CUDA_OK(cudaMalloc(&l.u, bytes)) ||
-        !STS_CUDA_OK(cudaMalloc(&l.t, bytes)) || !STS_CUDA_OK(cudaMalloc(&l.axf, l.nx * sizeof(double))) ||
-        !STS_CUDA_OK(cudaMalloc(&l.ayf, l.ny * sizeof(double))) ||
-        !STS_CUDA_OK(cudaMemcpy(l.axf, l.hax.data(), l.nx * sizeof(double), cudaMemcpyHostToDevice)) ||
-        !STS_CUDA_OK(cudaMemcpy(l.ayf, l.hay.data(), l.ny * sizeof(double), cudaMemcpyHostToDevice)))
-    {
-      mg->L.push_back(l);
-      return false;
-    }
     mg->L.push_back(l);
     if (l.dir < 0) break;
   }
-  return mg->L.back().dir < 0;
+  return mg->L.back().dir < 0 && pfmg_alloc(mg);
 }
 
 static bool pfmg_build(STS_PFMG mg, double gamma)
@@ -406,18 +589,14 @@ static bool pfmg_build(STS_PFMG mg, double gamma)
     if (l.nx > 2 && (l.ax >= l.ay || l.ny <= 2)) l.dir = 0;
     else if (l.ny > 2) l.dir = 1;
     else l.dir = -1;
-    const size_t bytes = (size_t)(l.nx * l.ny) * sizeof(double);
-    if (!STS_CUDA_OK(cudaMalloc(&l.f, bytes)) || !STS_CUDA_OK(cudaMalloc(&l.u, bytes)) ||
-        !STS_CUDA_OK(cudaMalloc(&l.t, bytes)))
-      return false;
     mg->L.push_back(l);
     if (l.dir < 0) break;
   }
-  return mg->L.back().dir < 0;
+  return mg->L.back().dir < 0 && pfmg_alloc(mg);
 }
 
 // smoothing sweeps on level l (u holds the iterate; Jacobi ping-pongs through t and copies back)
-static void pfmg_smooth(STS_PFMG mg, PfmgLevel& l, int sweeps, bool post, cudaStream_t st)
+static void pfmg_smooth(STS_PFMG mg, PfmgLevel& l, int sweeps, bool post, cudaStream_t st, bool zero_guess = false)
 {
   const dim3 b(32, 8);
   if (mg->periodic)
@@ -446,13 +625,15 @@ static void pfmg_smooth(STS_PFMG mg, PfmgLevel& l, int sweeps, bool post, cudaSt
     if (nw & 1) cudaMemcpyAsync(l.u, l.t, bytes, cudaMemcpyDeviceToDevice, st);
     return;
   }
+  const bool soft = l.nx * l.ny >= SOFT_POINTS;
   if (mg->relax == 1)
   {
     for (int s = 0; s < sweeps; ++s)
     {
       const double* in = (s & 1) ? l.t : l.u;
       double* out      = (s & 1) ? l.u : l.t;
-      jacobi_kernel<<<blocks2d(l.nx, l.ny, b), b, 0, st>>>(l.nx, l.ny, l.ax, l.ay, l.d, l.wd, l.f, in, out);
+      (soft ? jacobi_kernel<true> : jacobi_kernel<false>)<<<blocks2d(l.nx, l.ny, b), b, 0, st>>>(l.nx, l.ny, l.ax, l.ay,
+                                                                                           l.d, l.wd, l.f, in, out);
     }
     if (sweeps & 1) cudaMemcpyAsync(l.u, l.t, (size_t)(l.nx * l.ny) * sizeof(double), cudaMemcpyDeviceToDevice, st);
   }
@@ -462,10 +643,15 @@ static void pfmg_smooth(STS_PFMG mg, PfmgLevel& l, int sweeps, bool post, cudaSt
     for (int s = 0; s < sweeps; ++s)
       for (int h = 0; h < 2; ++h)
       {
+        if (zero_guess && s == 0 && h == 0)
+        {
+          (soft ? red_first_kernel<true> : red_first_kernel<false>)<<<g, b, 0, st>>>(l.nx, l.ny, l.dinv, l.f, l.u);
+          continue;
+        }
         // red then black before; after: black then red (relax 2, symmetric) or red then black
         // again (relax 3, nonsymmetric)
         const int color = (post && mg->relax == 2) ? 1 - h : h;
-        rbgs_kernel<<<g, b, 0, st>>>(l.nx, l.ny, l.ax, l.ay, l.dinv, l.f, l.u, color);
+        (soft ? rbgs_kernel<true> : rbgs_kernel<false>)<<<g, b, 0, st>>>(l.nx, l.ny, l.ax, l.ay, l.dinv, l.f, l.u, color);
       }
   }
 }
@@ -475,16 +661,18 @@ static void pfmg_vcycle(STS_PFMG mg, cudaStream_t st)
 {
   const dim3 b(32, 8);
   const int nl = (int)mg->L.size();
-  for (int lev = 0; lev < nl; ++lev)
+  int bottom   = nl - 1; // the first level of the one-block end
+  while (bottom > 0 && nl - bottom < BOTTOM_LEVELS && mg->L[bottom - 1].nx * mg->L[bottom - 1].ny <= BOTTOM_POINTS)
+    --bottom;
+  if (mg->L[bottom].nx * mg->L[bottom].ny > BOTTOM_POINTS) bottom = nl;
+  for (int lev = 0; lev < std::min(bottom, nl); ++lev)
   {
-    PfmgLevel& l = mg->L[lev];
-    cudaMemsetAsync(l.u, 0, (size_t)(l.nx * l.ny) * sizeof(double), st);
-    if (l.dir < 0)
-    {
-      pfmg_smooth(mg, l, PFMG_COARSE_SWEEPS, false, st);
-      break;
-    }
-    pfmg_smooth(mg, l, mg->nrelax, false, st);
+    PfmgLevel& l        = mg->L[lev];
+    const int sweeps    = l.dir < 0 ? PFMG_COARSE_SWEEPS : mg->nrelax;
+    const bool in_place = !mg->periodic && mg->relax != 1; // red/black sweeps in u
+    if (!in_place) cudaMemsetAsync(l.u, 0, (size_t)(l.nx * l.ny) * sizeof(double), st);
+    pfmg_smooth(mg, l, sweeps, false, st, in_place);
+    if (l.dir < 0) break;
     PfmgLevel& c = mg->L[lev + 1];
     if (mg->periodic)
     {
@@ -492,16 +680,40 @@ static void pfmg_vcycle(STS_PFMG mg, cudaStream_t st)
       per_restrict_kernel<<<blocks2d(c.nx, c.ny, b), b, 0, st>>>(l.nx, l.ny, l.dir, c.nx, c.ny, l.t, c.f);
       continue;
     }
-    residual_kernel<<<blocks2d(l.nx, l.ny, b), b, 0, st>>>(l.nx, l.ny, l.ax, l.ay, l.d, l.f, l.u, l.t);
-    restrict_kernel<<<blocks2d(c.nx, c.ny, b), b, 0, st>>>(l.nx, l.ny, l.dir, c.nx, c.ny, l.t, c.f);
+    // rows per thread only where the grid has them to spare
+    const dim3 g1 = blocks2d(c.nx, c.ny, b), g4 = blocks2d(c.nx, (c.ny + 3) / 4, b);
+    if (l.nx * l.ny >= SOFT_POINTS)
+      residual_restrict_kernel<4, true><<<g4, b, 0, st>>>(l.nx, l.ny, l.ax, l.ay, l.d, l.dir, c.nx, c.ny, l.f, l.u, c.f);
+    else
+      residual_restrict_kernel<1, false><<<g1, b, 0, st>>>(l.nx, l.ny, l.ax, l.ay, l.d, l.dir, c.nx, c.ny, l.f, l.u, c.f);
   }
-  for (int lev = nl - 2; lev >= 0; --lev)
+  if (bottom < nl)
+  {
+    BottomArgs B;
+    B.nl     = nl - bottom;
+    B.relax  = mg->relax;
+    B.nrelax = mg->nrelax;
+    for (int v = 0; v < B.nl; ++v)
+    {
+      const PfmgLevel& l = mg->L[bottom + v];
+      B.l[v] = {(int)l.nx, (int)l.ny, l.dir, l.ax, l.ay, l.d, l.dinv, l.wd, l.f, l.u, l.t, l.axf, l.ayf};
+    }
+    if (mg->periodic) bottom_kernel<true><<<1, BOTTOM_POINTS, 0, st>>>(B);
+    else bottom_kernel<false><<<1, BOTTOM_POINTS, 0, st>>>(B);
+  }
+  for (int lev = std::min(bottom, nl - 1) - 1; lev >= 0; --lev)
   {
     PfmgLevel& l = mg->L[lev];
     const PfmgLevel& c = mg->L[lev + 1];
     if (mg->periodic)
       per_prolong_kernel<<<blocks2d(l.nx, l.ny, b), b, 0, st>>>(l.nx, l.ny, l.dir, c.nx, c.ny, c.u, l.u);
-    else prolong_kernel<<<blocks2d(l.nx, l.ny, b), b, 0, st>>>(l.nx, l.ny, l.dir, c.nx, c.ny, c.u, l.u);
+    else
+    {
+      // the first half sweep after it: color 1 (relax 2) or 0 (relax 3), Jacobi reads every point
+      const int keep = mg->relax == 1 ? -1 : (mg->relax == 2 ? 0 : 1);
+      prolong_kernel<<<blocks2d(keep < 0 ? l.nx : (l.nx + 1) / 2, l.ny, b), b, 0, st>>>(l.nx, l.ny, l.dir, c.nx, c.ny,
+                                                                                        c.u, l.u, keep);
+    }
     pfmg_smooth(mg, l, mg->nrelax, true, st);
   }
 }
@@ -619,14 +831,24 @@ namespace {
 struct ShiftOp {
   STS_Problem p;
   double gamma;
-  N_Vector tmp;
 };
+// z = v - gamma A v, the operations of STS_JacTimes and N_VLinearSum(1, v, -gamma, A v) in one pass
+__global__ void shift_kernel(ProbDev P, double gamma, const double* __restrict__ v, double* __restrict__ z)
+{
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const long long j = (long long)blockIdx.y * blockDim.y + threadIdx.y;
+  if (i >= P.nx || j >= P.ny) return;
+  const double t = P.kind == STS_PROBLEM_PERIODIC ? periodic_point(P, v, i, j) : dirichlet_point(P, v, i, j);
+  z[j * P.nx + i] = __dadd_rn(v[j * P.nx + i], s64_mul(-gamma, t));
+}
 int shift_atimes(void* d, N_Vector v, N_Vector z)
 {
   ShiftOp* a = (ShiftOp*)d;
-  if (STS_JacTimes(v, a->tmp, 0.0, nullptr, nullptr, a->p, nullptr)) return -1;
-  N_VLinearSum_Sts(1.0, v, -a->gamma, a->tmp, z);
-  return 0;
+  if (NVL(v) != a->p->nx * a->p->ny || NVL(z) != NVL(v)) return -1;
+  const dim3 b(32, 8);
+  ctx_activate(a->p->ctx);
+  shift_kernel<<<blocks2d(a->p->nx, a->p->ny, b), b, 0, a->p->ctx->stream>>>(a->p->dev, a->gamma, NVD(v), NVD(z));
+  return STS_CUDA_OK(cudaGetLastError()) ? 0 : -1;
 }
 } // namespace
 
@@ -638,13 +860,12 @@ extern "C" int STS_ImplicitSolvePFMG(STS_Problem p, double gamma, STS_PFMG mg, N
   if (STS_PFMGPSetup(0.0, nullptr, nullptr, 0, nullptr, gamma, mg) != 0) return -1;
   void* LS = STS_SUNLinSol_PCG(b, STS_PREC_RIGHT, maxit, p->ctx);
   if (!LS) return -1;
-  ShiftOp op{p, gamma, N_VClone_Sts(b)};
+  ShiftOp op{p, gamma};
   STS_SUNLinSolSetATimes(LS, &op, shift_atimes);
   STS_SUNLinSolSetPreconditioner(LS, mg, STS_PFMGPrecSolve);
   const int rc = STS_SUNLinSolSolve(LS, x, b, tol);
   if (iters) *iters = STS_SUNLinSolNumIters(LS);
   if (relres) *relres = STS_SUNLinSolResNorm(LS);
   STS_SUNLinSolFree(LS);
-  N_VDestroy_Sts(op.tmp);
   return rc;
 }

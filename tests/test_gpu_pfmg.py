@@ -167,3 +167,21 @@ def test_cli_dirk_pfmg(stslib):
         assert abs(err - base[0]) <= 1e-6 * base[0]
         if k:
             assert its < base[1]
+
+
+@pytest.mark.parametrize("relax", [1, 2, 3])
+@pytest.mark.parametrize("kind,nx,ny,ky", [(1, 33, 31, 0.3), (1, 64, 16, 1.0), (1, 65, 63, 0.02), (1, 725, 724, 0.5),
+                                           (2, 32, 32, 0.5), (2, 66, 34, 0.5), (2, 33, 62, 0.1)])
+def test_vcycle_at_the_level_size_rules_bitwise(ctx, stslib, oracle, relax, kind, nx, ny, ky):
+    """One V-cycle with level sizes on both sides of the rules (the one-block end below 1025 points,
+    integer products and four coarse rows per thread from 2^19 points), ragged, both problems and all
+    relaxations, against the oracle bit for bit."""
+    pk = dict(kind=kind, nx=nx, ny=ny, kx=1.0, ky=ky, inhomogeneous=kind == 2)
+    G, O = stslib.Problem(ctx, **pk), oracle.Problem(**pk)
+    gamma = 0.01
+    r = np.random.default_rng(nx + ny).standard_normal(nx * ny)
+    mg = stslib.PFMG(G, relax=relax)
+    mg.setup(gamma)
+    z = G.vector()
+    mg.psolve(stslib.NVector.from_numpy(ctx, r), z, gamma)
+    assert np.array_equal(z.numpy(), O.pfmg_vcycle(gamma, r, relax=relax, nrelax=2)[0])
