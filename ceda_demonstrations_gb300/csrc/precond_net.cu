@@ -15,8 +15,8 @@
 // (rows+2) x (64+2) pixel tile in shared memory (16-byte halves XOR-swizzled by pixel so
 // ldmatrix is conflict-free), each warp computes 16-pixel x 16-channel tiles over the nine
 // taps with the weights held in registers as MMA fragments. A transposed convolution is the
-// same kernel with the flipped, transposed weights; the weight gradient is a per-tile FP32
-// reduction added to global memory with atomics.
+// same kernel with the flipped, transposed weights; the weight gradient contracts over the pixels
+// with the same MMA and adds the CTAs' sums in a fixed order.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -1291,52 +1291,140 @@ __global__ void __launch_bounds__(256) pair_meta_kernel(const float* __restrict_
   }
 }
 
-// weight gradient: dW[co][ci][tap] += sum_p g[p][co] * x[p + tap - 1][ci] over every image
-// of the batch. Each CTA walks 16 x 16 tiles (grid-stride over tiles of all images), keeps
-// its partial sums in registers and adds them to dW with one atomicAdd per weight.
-__global__ void __launch_bounds__(256) wgrad_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ g,
-                                                   int H, int W, int nimg, float* __restrict__ dW)
+// weight gradient: dW[co][ci][tap] = sum_p g[p][co] * x[p + tap - 1][ci] over every image of the
+// batch, a contraction over pixels: per tap a 16 x 16 product with K = pixels, on the tensor cores
+// (mma.sync m16n8k16 BF16 -> FP32; 16 rows are too few for a tcgen05 tile). Each CTA walks 16 x 16
+// tiles (grid-stride over tiles of all images, the next tile fetched by cp.async meanwhile); a warp
+// takes two rows of a tile, 16 pixels per step: both operands by transposing ldmatrix from the
+// pixel-major tile, the nine taps as shifts of the x rows' addresses, 72 sums per thread in
+// registers. The warps' sums are added in warp order and stored per CTA; wgrad_sum_kernel adds the
+// CTAs' in a fixed order, so a gradient does not depend on the order in which CTAs finish.
+// Bound by the tile traffic. 32 images of 128^2: 22.5 us (one (co, ci) pair per thread on the FP32
+// units, atomics: 114), 16 images of 64^2 12.3 (36); relative error against 64 bits 2.3e-7 (4.8e-7).
+constexpr int WG_T = 16; // tile edge
+__global__ void __launch_bounds__(256, 2) wgrad_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ g,
+                                                      int H, int W, int nimg, float* __restrict__ part)
 {
-  __shared__ float xs[18][18][CH];
-  __shared__ float gs[16][16][CH];
-  const int tid = threadIdx.x;
-  const int tx_n = (W + 15) / 16, ty_n = (H + 15) / 16;
+  constexpr int XR = (WG_T + 2) * 32, GR = WG_T * 32; // bytes of a tile row
+  __shared__ __align__(128) unsigned char xs[2][(WG_T + 2) * XR];
+  __shared__ __align__(128) unsigned char gs[2][WG_T * GR];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tx_n = (W + WG_T - 1) / WG_T, ty_n = (H + WG_T - 1) / WG_T;
   const long long ntiles = (long long)tx_n * ty_n * nimg;
-  // 2304 weights / 256 threads = 9 per thread: thread -> (co, ci) pair, all 9 taps
-  const int co = tid / CH, ci = tid % CH;
-  float acc[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-  for (long long tl = blockIdx.x; tl < ntiles; tl += gridDim.x)
-  {
+  auto fill = [&](int st, long long tl) {
     const int img = (int)(tl / ((long long)tx_n * ty_n));
     const int rem = (int)(tl % ((long long)tx_n * ty_n));
-    const int x0 = (rem % tx_n) * 16, y0 = (rem / tx_n) * 16;
+    const int x0 = (rem % tx_n) * WG_T, y0 = (rem / tx_n) * WG_T;
     const __nv_bfloat16* xi = x + (long long)img * H * W * CH;
     const __nv_bfloat16* gi = g + (long long)img * H * W * CH;
-    __syncthreads(); // previous tile consumed
-    for (int k = tid; k < 18 * 18 * CH; k += 256)
+    for (int k = tid; k < (WG_T + 2) * (WG_T + 2) * 2; k += 256)
     {
-      const int c = k % CH, px = (k / CH) % 18, py = k / (CH * 18);
+      const int h = k & 1, q = k >> 1, px = q % (WG_T + 2), py = q / (WG_T + 2);
       const int gx = x0 + px - 1, gy = y0 + py - 1;
-      xs[py][px][c] = (gx >= 0 && gx < W && gy >= 0 && gy < H) ? __bfloat162float(xi[((long long)gy * W + gx) * CH + c]) : 0.f;
+      const bool in = gx >= 0 && gx < W && gy >= 0 && gy < H;
+      cp_async16(smem_u32(xs[st] + py * XR + swz(px, h)), in ? xi + ((long long)gy * W + gx) * CH + h * 8 : x, in);
     }
-    for (int k = tid; k < 16 * 16 * CH; k += 256)
+    for (int k = tid; k < WG_T * WG_T * 2; k += 256)
     {
-      const int c = k % CH, px = (k / CH) % 16, py = k / (CH * 16);
+      const int h = k & 1, q = k >> 1, px = q % WG_T, py = q / WG_T;
       const int gx = x0 + px, gy = y0 + py;
-      gs[py][px][c] = (gx < W && gy < H) ? __bfloat162float(gi[((long long)gy * W + gx) * CH + c]) : 0.f;
+      const bool in = gx < W && gy < H;
+      cp_async16(smem_u32(gs[st] + py * GR + swz(px, h)), in ? gi + ((long long)gy * W + gx) * CH + h * 8 : g, in);
     }
-    __syncthreads();
-    for (int py = 0; py < 16; ++py)
-      for (int px = 0; px < 16; ++px)
-      {
-        const float gv = gs[py][px][co];
-#pragma unroll
-        for (int t = 0; t < 9; ++t) acc[t] = fmaf(gv, xs[py + t / 3][px + t % 3][ci], acc[t]);
-      }
-  }
+    cp_async_commit();
+  };
+  float acc[9][2][4];
 #pragma unroll
   for (int t = 0; t < 9; ++t)
-    if (acc[t] != 0.f) atomicAdd(&dW[(co * CH + ci) * 9 + t], acc[t]);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) acc[t][k >> 2][k & 3] = 0.f;
+  // ldmatrix row addresses of this lane: matrix lane / 8, row lane % 8
+  const int mi = lane >> 3, r = lane & 7;
+  const int ga = swz((mi >> 1) * 8 + r, mi & 1); // A: pixels 0-7 / 8-15, the channel halves as row blocks
+  int xa[3];                                     // B: pixel halves as k blocks, channel halves as n blocks
+#pragma unroll
+  for (int dx = 0; dx < 3; ++dx) xa[dx] = swz((mi & 1) * 8 + r + dx, mi >> 1);
+  auto ldsm = [](uint32_t (&v)[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3])
+                 : "r"(addr)
+                 : "memory");
+  };
+  int st = 0;
+  if (blockIdx.x < ntiles) fill(0, blockIdx.x);
+  for (long long tl = blockIdx.x; tl < ntiles; tl += gridDim.x, st ^= 1)
+  {
+    if (tl + gridDim.x < ntiles) fill(st ^ 1, tl + gridDim.x);
+    else cp_async_commit();
+    cp_async_wait1();
+    __syncthreads();
+#pragma unroll 1
+    for (int py = 2 * warp; py < 2 * warp + 2; ++py)
+    {
+      uint32_t av[4];
+      ldsm(av, smem_u32(gs[st] + py * GR) + ga);
+#pragma unroll
+      for (int t = 0; t < 9; ++t)
+      {
+        uint32_t bv[4];
+        ldsm(bv, smem_u32(xs[st] + (py + t / 3) * XR) + xa[t % 3]);
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+                       "{%0,%1,%2,%3};"
+                       : "+f"(acc[t][h][0]), "+f"(acc[t][h][1]), "+f"(acc[t][h][2]), "+f"(acc[t][h][3])
+                       : "r"(av[0]), "r"(av[1]), "r"(av[2]), "r"(av[3]), "r"(bv[2 * h]), "r"(bv[2 * h + 1]));
+      }
+    }
+    __syncthreads(); // tile consumed
+  }
+  cp_async_wait0();
+  __syncthreads();
+  // the warps' sums, in warp order
+  float* sum = reinterpret_cast<float*>(xs); // WSZ floats
+  static_assert(sizeof(xs) >= WSZ * sizeof(float), "sum buffer");
+  const int co = lane >> 2, ci = (lane & 3) * 2;
+  for (int w = 0; w < 8; ++w)
+  {
+    if (warp == w)
+#pragma unroll
+      for (int t = 0; t < 9; ++t)
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+        { // accumulator k of a tap: row co (+ 8), column ci (+ 1) of channel half k / 4
+          float* d = &sum[((co + ((k & 2) ? 8 : 0)) * CH + (k >> 2) * 8 + ci + (k & 1)) * 9 + t];
+          *d       = w == 0 ? acc[t][k >> 2][k & 3] : *d + acc[t][k >> 2][k & 3];
+        }
+    __syncthreads();
+  }
+  for (int k = tid; k < WSZ; k += 256) part[(long long)blockIdx.x * WSZ + k] = sum[k];
+}
+
+// g += the CTAs' sums of the layer's two weight-gradient passes: 32 weights per block, 16 threads
+// each, their sums added in order (8 us for the eight passes of a minibatch of 32 at 128^2)
+constexpr int WG_PASSES = 2 * NLAYER; // a layer's weights are used twice
+struct WgradParts {
+  int layer[WG_PASSES], blocks[WG_PASSES];
+};
+__global__ void __launch_bounds__(512) wgrad_sum_kernel(WgradParts q, int stride, const float* __restrict__ part,
+                                                       float* __restrict__ g)
+{
+  __shared__ float s[16][32];
+  const int c = threadIdx.x & 31, y = threadIdx.x >> 5;
+  const int k = blockIdx.x * 32 + c, l = k / WSZ, wk = k % WSZ;
+  float v = 0.f;
+  for (int p = 0; p < WG_PASSES; ++p)
+    if (q.layer[p] == l)
+    {
+      const float* src = part + (long long)p * stride * WSZ + wk;
+#pragma unroll 4
+      for (int b = y; b < q.blocks[p]; b += 16) v += src[(long long)b * WSZ];
+    }
+  s[y][c] = v;
+  __syncthreads();
+  if (y) return;
+  for (int r = 1; r < 16; ++r) v += s[r][c];
+  g[k] += v;
 }
 
 // Adam on FP32 master weights; mask keeps padded entries at zero; writes the BF16 copy
@@ -1439,6 +1527,7 @@ struct STS_Net_ {
   float* w        = nullptr; // FP32 master weights, 9 x 2304
   float* mask     = nullptr;
   float *m = nullptr, *v = nullptr, *g = nullptr;
+  float* wpart = nullptr; // the weight-gradient CTAs' sums (training only)
   uint2* wf       = nullptr; // forward fragments, 9 x 576
   uint2* wt       = nullptr; // input-gradient fragments
   __nv_bfloat16* wu  = nullptr; // forward UMMA B operands (tcgen05 inference), 9 x 256 per layer
@@ -1492,6 +1581,15 @@ static void free_levels(STS_Net nt)
 }
 
 // activation buffers for `pix` level-0 pixels (a batch of images of one size)
+// room for the weight-gradient CTAs' sums of one backward pass (22 MB)
+static int wgrad_blocks(STS_Net nt);
+static bool ensure_wpart(STS_Net nt)
+{
+  bool ok = true;
+  if (!nt->wpart) nt->wpart = (float*)dalloc((size_t)net::WG_PASSES * wgrad_blocks(nt) * WSZ * 4, &ok);
+  return ok;
+}
+
 static bool ensure_capacity(STS_Net nt, long long pix)
 {
   if (pix <= nt->cap) return true;
@@ -1690,6 +1788,7 @@ extern "C" int STS_NetFree(STS_Net* pn)
   cudaFree(nt->m);
   cudaFree(nt->v);
   cudaFree(nt->g);
+  cudaFree(nt->wpart);
   cudaFree(nt->wf);
   cudaFree(nt->wu);
   cudaFree(nt->wut);
@@ -1934,11 +2033,18 @@ static void net_forward_infer(STS_Net nt, int n, const double* r, double scale, 
   conv_launch<2, net::LD_UPADD>(nt, L[0].h, n, 1, nt->wt + net::L_IN * 576, nullptr, zout, out_scale, nullptr, lu); // z
 }
 
-static void wgrad(STS_Net nt, const __nv_bfloat16* x, const __nv_bfloat16* g, int n, int nimg, int layer)
+// CTAs of a weight-gradient pass: two per SM (their registers), a tile at least each
+static int wgrad_blocks(STS_Net nt) { return 2 * nt->ctx->num_sms; }
+
+// one weight-gradient pass, its CTAs' sums into the pass's part of nt->wpart
+static void wgrad(STS_Net nt, net::WgradParts& q, int pass, const __nv_bfloat16* x, const __nv_bfloat16* g, int n, int nimg,
+                  int layer)
 {
-  const long long tiles = (long long)((n + 15) / 16) * ((n + 15) / 16) * nimg;
-  const int grid        = (int)std::min<long long>(tiles, 2LL * nt->ctx->num_sms);
-  net::wgrad_kernel<<<grid, 256, 0, nt->ctx->stream>>>(x, g, n, n, nimg, nt->g + layer * WSZ);
+  const long long t = (n + net::WG_T - 1) / net::WG_T;
+  const int grid    = (int)std::min<long long>(t * t * nimg, wgrad_blocks(nt));
+  q.layer[pass]     = layer;
+  q.blocks[pass]    = grid;
+  net::wgrad_kernel<<<grid, 256, 0, nt->ctx->stream>>>(x, g, n, n, nimg, nt->wpart + (size_t)pass * wgrad_blocks(nt) * WSZ);
 }
 
 // out_fine += 0.25 up(coarse) (adjoint of the 2x2 mean), fine at n x n
@@ -1959,30 +2065,32 @@ static void net_backward(STS_Net nt, int n, int nimg, const float* e, double gsc
   net::Level* L   = nt->L;
   const long long ip = (long long)n * n, np = ip * nimg;
   const int m = nimg;
+  net::WgradParts q;
   net::gradz_kernel<<<grid_for(np), 256, 0, st>>>(np, n, nt->z, e, gscale, meta, L[0].dy, nt->dacc); // d gx (3 ch)
   // adjoint pass, top (level 0) to bottom (level 3)
-  wgrad(nt, L[0].dy, L[0].g, n, m, net::L_IN);                 // W_in via convT(g0)
+  wgrad(nt, q, 0, L[0].dy, L[0].g, n, m, net::L_IN);                 // W_in via convT(g0)
   conv(nt, L[0].dy, n, m, net::L_IN, false, L[0].dg);          // d g0 (= d h0 so far)
   pool(nt, L[0].dg, n, m, L[1].dy);                            // d y1
-  wgrad(nt, L[1].dy, L[1].g, n / 2, m, net::L_1);
+  wgrad(nt, q, 1, L[1].dy, L[1].g, n / 2, m, net::L_1);
   conv(nt, L[1].dy, n / 2, m, net::L_1, false, L[1].dg);       // d g1 (= d h1 so far)
   pool(nt, L[1].dg, n / 2, m, L[2].dy);                        // d y2
-  wgrad(nt, L[2].dy, L[2].g, n / 4, m, net::L_2);
+  wgrad(nt, q, 2, L[2].dy, L[2].g, n / 4, m, net::L_2);
   conv(nt, L[2].dy, n / 4, m, net::L_2, false, L[2].dg);       // d g2 (= d h2 so far)
   pool(nt, L[2].dg, n / 4, m, L[3].dy);                        // d y3
-  wgrad(nt, L[3].dy, L[3].h, n / 8, m, net::L_3);              // g3 = h3
+  wgrad(nt, q, 3, L[3].dy, L[3].h, n / 8, m, net::L_3);              // g3 = h3
   conv(nt, L[3].dy, n / 8, m, net::L_3, false, L[3].dg);       // d h3
   // encoder, bottom to top
-  wgrad(nt, L[3].p, L[3].dg, n / 8, m, net::L_3);
+  wgrad(nt, q, 4, L[3].p, L[3].dg, n / 8, m, net::L_3);
   conv(nt, L[3].dg, n / 8, m, net::L_3, true, L[3].t);
   poolT_add(nt, L[3].t, n / 4, m, L[2].dg);                    // d h2 += poolT(convT(d h3))
-  wgrad(nt, L[2].p, L[2].dg, n / 4, m, net::L_2);
+  wgrad(nt, q, 5, L[2].p, L[2].dg, n / 4, m, net::L_2);
   conv(nt, L[2].dg, n / 4, m, net::L_2, true, L[2].t);
   poolT_add(nt, L[2].t, n / 2, m, L[1].dg);                    // d h1
-  wgrad(nt, L[1].p, L[1].dg, n / 2, m, net::L_1);
+  wgrad(nt, q, 6, L[1].p, L[1].dg, n / 2, m, net::L_1);
   conv(nt, L[1].dg, n / 2, m, net::L_1, true, L[1].t);
   poolT_add(nt, L[1].t, n, m, L[0].dg);                        // d h0
-  wgrad(nt, L[0].x, L[0].dg, n, m, net::L_IN);
+  wgrad(nt, q, 7, L[0].x, L[0].dg, n, m, net::L_IN);
+  net::wgrad_sum_kernel<<<NLAYER * WSZ / 32, 512, 0, st>>>(q, wgrad_blocks(nt), nt->wpart, nt->g);
 }
 
 static bool net_size_ok(STS_Net nt, int n)
@@ -2044,6 +2152,7 @@ extern "C" int STS_NetLossGrad(STS_Net nt, int n, const double* r, const float* 
     const double so = j > 0 ? eh[q - n] : 0.0, no = j < n - 1 ? eh[q + n] : 0.0;
     eMe += c * ((1.0 + 2.0 * (gcx + gcy)) * c - gcx * (w + ea) - gcy * (so + no));
   }
+  if (!ensure_wpart(nt)) return -1;
   if (!nt->mb)
   {
     bool ok = true;
@@ -2081,7 +2190,7 @@ extern "C" int STS_NetTrain(STS_Net nt, int n, int nsamples, const float* r, con
   cudaStream_t st = nt->ctx->stream;
   const long long ip = (long long)n * n;
   batch = std::min(batch, nsamples);
-  if (!ensure_capacity(nt, ip * batch)) return -1;
+  if (!ensure_capacity(nt, ip * batch) || !ensure_wpart(nt)) return -1;
   cudaFree(nt->mb);
   cudaFree(nt->idx);
   nt->mb  = nullptr;

@@ -133,6 +133,26 @@ def test_gradients_match_oracle(ctx, weights):
         assert not np.any(grad[nm][co:]) and not np.any(grad[nm][:, ci:])
 
 
+@pytest.mark.parametrize("n", [16, 48, 144])
+def test_gradients_on_partial_tiles(ctx, weights, n):
+    """Sizes whose levels end inside a 16 x 16 tile (n/8 = 2, 6, 18), against the oracle with the
+    tolerance above; sums are taken in a fixed order, so a second call gives the same bits."""
+    rng = np.random.default_rng(n)
+    r = rng.standard_normal((n, n))
+    e = rng.standard_normal((n, n)).astype(np.float32)
+    net = sts.Net(ctx, n, seed=0)
+    net.set_weights(weights)
+    rv, et = sts.NVector.from_numpy(ctx, r), _f32_dev(e)
+    args = (n, rv.ptr, et.data_ptr(), 0.4, -0.2, 0.5, 24.0, 3.0)
+    _, grad = net.loss_grad(*args)
+    _, again = net.loss_grad(*args)
+    _, gref = convnet.loss_and_grad(weights, r, e.astype(np.float64), 0.4, -0.2, 0.5, 24.0, 3.0)
+    for nm in convnet.NAMES:
+        co, ci = convnet.shape(nm)[:2]
+        assert _rel(grad[nm][:co, :ci], gref[nm]) < GRAD_TOL, nm
+        assert np.array_equal(grad[nm], again[nm])
+
+
 def _harvest(ctx, n, ky, gam_rel, crop, ncrops, every, max_pairs, seed):
     p = sts.Problem(ctx, sts.UNFORCED, n, n, 1.0, ky)
     dx = 1.0 / (n + 1)
