@@ -79,9 +79,11 @@ struct STS_Batch_ {
   double big_share = 0.0;      // estimated cost share of the clustered group
   int* dorder_big   = nullptr; // cost-ordered indices of each group
   int* dorder_small = nullptr;
-  cudaStream_t side = nullptr; // second stream for the single-CTA group
-  cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+  std::vector<int> order_big;  // dorder_big on the host
+  cudaStream_t side[2] = {};   // streams for the groups beside the first one
+  cudaEvent_t ev_fork = nullptr, ev_join[2] = {};
   std::vector<double> cost;
+  double cost_total = 0.0;
 };
 
 // ---------------------------------------------------------------------------------------
@@ -205,22 +207,158 @@ __device__ double inst_exact_sum(xsum::Limbs& a, unsigned flags, long long (*sm)
 // Stencil-row load: rows owned by another CTA of the cluster are read through L2 (ld.cg),
 // so no stale L1 line of an earlier sweep is used.
 __device__ __forceinline__ double ldrow(const double* p, bool foreign) { return foreign ? __ldcg(p) : *p; }
-__device__ __forceinline__ float ldrowf(const float* p, bool foreign) { return foreign ? __ldcg(p) : *p; }
+__device__ __forceinline__ float ldrow(const float* p, bool foreign) { return foreign ? __ldcg(p) : *p; }
 
-__device__ __forceinline__ double lap(const double* __restrict__ u, int n, int i, int j, int j0, int j1, double cx,
-                                      double cy, double cc)
+// A u at one point from its row neighbours and column neighbours, in the oracle's order
+__device__ __forceinline__ double lap(double uc, double uw, double ue, double us, double un, double cx, double cy,
+                                      double cc)
 {
-  const long long k = (long long)j * n + i;
-  const double uc = u[k];
-  const double uw = (i > 0) ? u[k - 1] : 0.0;
-  const double ue = (i < n - 1) ? u[k + 1] : 0.0;
-  const double us = (j > 0) ? ldrow(&u[k - n], j - 1 < j0) : 0.0;
-  const double un = (j < n - 1) ? ldrow(&u[k + n], j + 1 >= j1) : 0.0;
-  const double sx = uw + ue, sy = us + un;
-  double acc      = cc * uc;
-  acc             = __fma_rn(cx, sx, acc);
-  acc             = __fma_rn(cy, sy, acc);
+  double acc = cc * uc;
+  acc        = __fma_rn(cx, uw + ue, acc);
+  acc        = __fma_rn(cy, us + un, acc);
   return acc;
+}
+
+// A sweep of a CTA over its rows [j0, j1): the 32-column tiles times S row strips are dealt to the
+// warps, S the smallest number that gives every warp the same count. f(i, a, b) marches rows
+// [a, b) of column i.
+template <int NW, typename F>
+__device__ __forceinline__ void sweep(int n, int j0, int j1, F&& f)
+{
+  const int T = (n + 31) >> 5, S = NW / min(NW, T & -T), R = (j1 - j0 + S - 1) / S;
+  for (int q = threadIdx.x >> 5; q < T * S; q += NW)
+  {
+    const int st = q / T, i = ((q - st * T) << 5) + (threadIdx.x & 31);
+    const int a = j0 + st * R, b = min(a + R, j1);
+    if (i < n && a < b) f(i, a, b);
+  }
+}
+
+// march rows [a, b) of column i of u: g(k, centre, west, east, south, north) per point
+template <typename T, typename G>
+__device__ __forceinline__ void march(const T* u, int n, int i, int a, int b, int j0, int j1, G&& g)
+{
+  long long k = (long long)a * n + i;
+  T up        = a > 0 ? ldrow(&u[k - n], a - 1 < j0) : T(0);
+  T cur       = u[k];
+#pragma unroll 1
+  for (int j = a; j < b; ++j, k += n)
+  {
+    const T dn = (j < n - 1) ? ldrow(&u[k + n], j + 1 >= j1) : T(0);
+    const T w  = (i > 0) ? u[k - 1] : T(0);
+    const T e  = (i < n - 1) ? u[k + 1] : T(0);
+    g(k, cur, w, e, up, dn);
+    up  = cur;
+    cur = dn;
+  }
+}
+
+// The sweeps that take the time are functions of their own, so that the integrator's state does
+// not sit in the registers of their loops (64 instances: 129 ms against 135). Operations stay
+// FP64 instructions: integer code (soft64.cuh) is slower where one CTA per SM is left (147 ms).
+#define BATCH_FN __device__ __noinline__
+
+// Y_j of one FP64 stage
+struct StageCoef {
+  double gc, gx, gy, gn, g0, gf;
+};
+template <int NW>
+BATCH_FN void stage_sweep(int n, int j0, int j1, StageCoef C, const double* ym1, const double* ym2, const double* yc,
+                          const double* F0, double* yj)
+{
+  sweep<NW>(n, j0, j1, [&](int i, int a, int b) {
+    march(ym1, n, i, a, b, j0, j1, [&](long long k, double c, double w, double e, double so, double no) {
+      const double m2 = ym2[k], z0 = yc[k], q0 = F0[k];
+      const double sx = w + e, sy = so + no;
+      double acc      = C.gc * c;
+      acc             = __fma_rn(C.gx, sx, acc);
+      acc             = __fma_rn(C.gy, sy, acc);
+      acc             = __fma_rn(C.gn, m2, acc);
+      acc             = __fma_rn(C.g0, z0, acc);
+      yj[k]           = __fma_rn(C.gf, q0, acc);
+    });
+  });
+}
+
+// d_j of one mixed stage; yn: y_new = y + d_s (last stage only)
+struct StageCoefF {
+  float gs, gx, gy, gm, gF;
+};
+template <int NW, bool M2, bool LAST>
+__device__ __forceinline__ void stage_sweep_f(int n, int j0, int j1, const StageCoefF& C, const float* dm1, const float* dm2,
+                                              const float* ff, float* dj, const double* yc, double* yn)
+{
+  sweep<NW>(n, j0, j1, [&](int i, int a, int b) {
+    march(dm1, n, i, a, b, j0, j1, [&](long long k, float c, float w, float e, float so, float no) {
+      const float m2 = M2 ? dm2[k] : 0.0f;
+      const float dv = mixed_point<false>(C.gs, C.gx, C.gy, C.gm, C.gF, c, w, e, so, no, m2, ff[k], 0.f, 0.f, 0.f, 0.f);
+      dj[k]          = dv;
+      if (LAST) yn[k] = yc[k] + s64_from_float(dv);
+    });
+  });
+}
+template <int NW>
+BATCH_FN void stage_sweep(int n, int j0, int j1, StageCoefF C, const float* dm1, const float* dm2, const float* ff,
+                          float* dj, const double* yc, double* yn)
+{
+  if (yn && dm2) stage_sweep_f<NW, true, true>(n, j0, j1, C, dm1, dm2, ff, dj, yc, yn);
+  else if (yn) stage_sweep_f<NW, false, true>(n, j0, j1, C, dm1, dm2, ff, dj, yc, yn);
+  else if (dm2) stage_sweep_f<NW, true, false>(n, j0, j1, C, dm1, dm2, ff, dj, yc, yn);
+  else stage_sweep_f<NW, false, false>(n, j0, j1, C, dm1, dm2, ff, dj, yc, yn);
+}
+
+// step end: F_new = A y_new, err = 0.8 (y - y_new) + 0.4 h (F + F_new); this thread's part of the
+// exact sum of the weighted squares
+template <int NW>
+BATCH_FN void end_sweep(int n, int j0, int j1, double cx, double cy, double cc, double p4h, double rtol, double atol,
+                        const double* yc, const double* F0, const double* Ys, double* Fnew, xsum::Limbs& out,
+                        unsigned& flags)
+{
+  xsum::Limbs ae;
+  xsum::zero(ae);
+  unsigned fe = 0;
+  sweep<NW>(n, j0, j1, [&](int i, int a, int b) {
+    march(Ys, n, i, a, b, j0, j1, [&](long long k, double c, double w, double ea, double so, double no) {
+      const double yv = yc[k], f0 = F0[k];
+      const double f  = lap(c, w, ea, so, no, cx, cy, cc);
+      Fnew[k]         = f;
+      double e        = 0.8 * (yv - c);
+      e               = __fma_rn(p4h, f0, e);
+      e               = __fma_rn(p4h, f, e);
+      const double wt = 1.0 / (rtol * fabs(yv) + atol);
+      const double x  = e * wt;
+      xsum::add(ae, x * x, fe);
+    });
+  });
+  out   = ae;
+  flags = fe;
+}
+
+// the same after mixed stages, y - y_new as -d_s (the single-problem form), and F_new in FP32
+template <int NW>
+BATCH_FN void end_sweep(int n, int j0, int j1, double cx, double cy, double cc, double p4h, double rtol, double atol,
+                        const double* yc, const double* F0, const double* yn, const float* ds, double* Fnew,
+                        float* Ffn, xsum::Limbs& out, unsigned& flags)
+{
+  xsum::Limbs ae;
+  xsum::zero(ae);
+  unsigned fe = 0;
+  sweep<NW>(n, j0, j1, [&](int i, int a, int b) {
+    march(yn, n, i, a, b, j0, j1, [&](long long k, double c, double w, double ea, double so, double no) {
+      const double yv = yc[k], f0 = F0[k];
+      const float dv  = ds[k];
+      const double f  = lap(c, w, ea, so, no, cx, cy, cc);
+      Fnew[k]         = f;
+      Ffn[k]          = s64_to_float(f);
+      double e        = 0.8 * -s64_from_float(dv);
+      e               = __fma_rn(p4h, f0, e);
+      e               = __fma_rn(p4h, f, e);
+      const double x  = e * mixed_weight(rtol, atol, yv);
+      xsum::add(ae, x * x, fe);
+    });
+  });
+  out   = ae;
+  flags = fe;
 }
 
 // CL CTAs (a thread-block cluster when CL > 1) integrate one instance together: CTA `rank`
@@ -264,7 +402,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) batch_kernel(BatchInst* __restr
     }
 #endif
     const double cx = I.cx, cy = I.cy, cc = I.cc, rho = I.rho;
-    // seven instance-local regions: the y array and six work regions; roles are indices.
+      // seven instance-local regions: the y array and six work regions; roles are indices.
     // FP64 stages: y, F, F_new and three Y stage buffers (regions 3-5). Mixed stages: y, F,
     // F_new, y_new (region 3) and, as FP32 arrays of N values, three increments d (regions 4
     // and 5) and the FP32 copies of F and F_new (region 5, second half, and region 6).
@@ -279,14 +417,13 @@ __global__ void __launch_bounds__(NT, 1024 / NT) batch_kernel(BatchInst* __restr
     float* Ff[2] = {reinterpret_cast<float*>(P[5]) + N, reinterpret_cast<float*>(P[6])};
 
     // F_0 = A y_0 (and its FP32 copy for the mixed stages)
-    for (int j = j0 + warp; j < j1; j += NW)
-      for (int i = lane; i < n; i += 32)
-      {
-        const long long k = (long long)j * n + i;
-        const double f    = lap(P[iy], n, i, j, j0, j1, cx, cy, cc);
-        P[iF][k]          = f;
-        if (MIXED) Ff[0][k] = (float)f;
-      }
+    sweep<NW>(n, j0, j1, [&](int i, int a, int b) {
+      march(P[0], n, i, a, b, j0, j1, [&](long long k, double c, double w, double e, double so, double no) {
+        const double f = lap(c, w, e, so, no, cx, cy, cc);
+        P[1][k]        = f;
+        if (MIXED) Ff[0][k] = s64_to_float(f);
+      });
+    });
     inst_sync<CL>();
     long long nfe = 1, nst = 0, natt = 0, netf = 0, nexp = 0, stmax = 0, sttot = 0, nhist = 0;
     double t = 0.0, hnext = 0.0, hlast = 0.0, ep1 = 0.0, ep2 = 0.0;
@@ -326,15 +463,14 @@ __global__ void __launch_bounds__(NT, 1024 / NT) batch_kernel(BatchInst* __restr
       xsum::Limbs a2;
       xsum::zero(a2);
       unsigned f2 = 0;
-      for (int j = j0 + warp; j < j1; j += NW)
-        for (int i = lane; i < n; i += 32)
-        {
-          const long long k = (long long)j * n + i;
-          const double f1v  = lap(y1, n, i, j, j0, j1, cx, cy, cc);
-          const double wt   = 1.0 / (prm.rtol * fabs(yc[k]) + prm.atol);
-          const double x    = (f1v - F0[k]) * wt;
+      sweep<NW>(n, j0, j1, [&](int i, int a, int b) {
+        march((const double*)y1, n, i, a, b, j0, j1, [&](long long k, double c, double w, double e, double so, double no) {
+          const double f1v = lap(c, w, e, so, no, cx, cy, cc);
+          const double wt  = 1.0 / (prm.rtol * fabs(yc[k]) + prm.atol);
+          const double x   = (f1v - F0[k]) * wt;
           xsum::add(a2, x * x, f2);
-        }
+        });
+      });
       nfe++;
       const double d2 = sqrt(inst_exact_sum<NT, CL>(a2, f2, sm, climb, &sflags, &sres) / (double)N) / h0;
       const double dm = d1 > d2 ? d1 : d2;
@@ -375,7 +511,6 @@ __global__ void __launch_bounds__(NT, 1024 / NT) batch_kernel(BatchInst* __restr
         const double* yc = P[iy];
         const double* F0 = P[iF];
         xsum::Limbs ae;
-        xsum::zero(ae);
         unsigned fe      = 0;
         const double p4h = 0.4 * h;
         int last         = 0; // FP64 stages: index into bufs of Y_{j-1}
@@ -408,20 +543,8 @@ __global__ void __launch_bounds__(NT, 1024 / NT) batch_kernel(BatchInst* __restr
             const float* ff  = Ff[iff];
             const int nxt    = (lastd + 1) % 3;
             float* dj        = D[nxt];
-            for (int j = j0 + warp; j < j1; j += NW)
-              for (int i = lane; i < n; i += 32)
-              {
-                const long long k = (long long)j * n + i;
-                const float dw = (i > 0) ? dm1[k - 1] : 0.0f;
-                const float de = (i < n - 1) ? dm1[k + 1] : 0.0f;
-                const float ds = (j > 0) ? ldrowf(&dm1[k - n], j - 1 < j0) : 0.0f;
-                const float dn = (j < n - 1) ? ldrowf(&dm1[k + n], j + 1 >= j1) : 0.0f;
-                const float m2 = dm2 ? dm2[k] : 0.0f;
-                const float dv = mixed_point<false>(gs, gx, gy, gm, gF, dm1[k], dw, de, ds, dn, m2, ff[k], 0.f, 0.f,
-                                                    0.f, 0.f);
-                dj[k] = dv;
-                if (jst == s) yn[k] = yc[k] + (double)dv; // the last stage also forms y_new = y + d_s
-              }
+            stage_sweep<NW>(n, j0, j1, StageCoefF{gs, gx, gy, gm, gF}, dm1, dm2, ff, dj, yc,
+                            jst == s ? yn : nullptr); // the last stage also forms y_new
             inst_sync<CL>();
             dm2   = dm1;
             lastd = nxt;
@@ -430,22 +553,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) batch_kernel(BatchInst* __restr
           const float* dsv = D[lastd];
           double* Fnew = P[iFn];
           float* Ffn   = Ff[1 - iff];
-          for (int j = j0 + warp; j < j1; j += NW)
-            for (int i = lane; i < n; i += 32)
-            {
-              const long long k = (long long)j * n + i;
-              const double f    = lap(yn, n, i, j, j0, j1, cx, cy, cc);
-              Fnew[k]           = f;
-              Ffn[k]            = (float)f;
-              const double yv   = yc[k];
-              const double d    = -(double)dsv[k]; // y_n - y_{n+1} as -d_s (the single-problem form)
-              double e          = 0.8 * d;
-              e                 = __fma_rn(p4h, F0[k], e);
-              e                 = __fma_rn(p4h, f, e);
-              const double wt   = mixed_weight(prm.rtol, prm.atol, yv);
-              const double x    = e * wt;
-              xsum::add(ae, x * x, fe);
-            }
+          end_sweep<NW>(n, j0, j1, cx, cy, cc, p4h, prm.rtol, prm.atol, yc, F0, yn, dsv, Fnew, Ffn, ae, fe);
         }
         else
         {
@@ -472,23 +580,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) batch_kernel(BatchInst* __restr
             const double* ym1 = P[bufs[last]];
             const int nxt     = (last + 1) % 3;
             double* yj        = P[bufs[nxt]];
-            for (int j = j0 + warp; j < j1; j += NW)
-              for (int i = lane; i < n; i += 32)
-              {
-                const long long k = (long long)j * n + i;
-                const double uw = (i > 0) ? ym1[k - 1] : 0.0;
-                const double ue = (i < n - 1) ? ym1[k + 1] : 0.0;
-                const double us = (j > 0) ? ldrow(&ym1[k - n], j - 1 < j0) : 0.0;
-                const double un = (j < n - 1) ? ldrow(&ym1[k + n], j + 1 >= j1) : 0.0;
-                const double sx = uw + ue, sy = us + un;
-                double acc      = gc * ym1[k];
-                acc             = __fma_rn(gx, sx, acc);
-                acc             = __fma_rn(gy, sy, acc);
-                acc             = __fma_rn(gn, ym2[k], acc);
-                acc             = __fma_rn(g0, yc[k], acc);
-                acc             = __fma_rn(gf, F0[k], acc);
-                yj[k]           = acc;
-              }
+            stage_sweep<NW>(n, j0, j1, StageCoef{gc, gx, gy, gn, g0, gf}, ym1, ym2, yc, F0, yj);
             inst_sync<CL>();
             ym2  = ym1;
             last = nxt;
@@ -496,21 +588,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) batch_kernel(BatchInst* __restr
           const double* Ys = P[bufs[last]];
           double* Fnew     = P[iFn];
           // step end: Fnew = A Ys, err = 0.8 (y - Ys) + 0.4 h (F + Fnew), exact WRMS
-          for (int j = j0 + warp; j < j1; j += NW)
-            for (int i = lane; i < n; i += 32)
-            {
-              const long long k = (long long)j * n + i;
-              const double f    = lap(Ys, n, i, j, j0, j1, cx, cy, cc);
-              Fnew[k]           = f;
-              const double yv   = yc[k];
-              const double d    = yv - Ys[k];
-              double e          = 0.8 * d;
-              e                 = __fma_rn(p4h, F0[k], e);
-              e                 = __fma_rn(p4h, f, e);
-              const double wt   = 1.0 / (prm.rtol * fabs(yv) + prm.atol);
-              const double x    = e * wt;
-              xsum::add(ae, x * x, fe);
-            }
+          end_sweep<NW>(n, j0, j1, cx, cy, cc, p4h, prm.rtol, prm.atol, yc, F0, Ys, Fnew, ae, fe);
         }
         const double dsm = sqrt(inst_exact_sum<NT, CL>(ae, fe, sm, climb, &sflags, &sres) / (double)N);
         nfe += s;
@@ -600,16 +678,14 @@ __global__ void __launch_bounds__(NT, 1024 / NT) batch_kernel(BatchInst* __restr
 // ---------------------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------------------
+// whether clusters of CL CTAs can run (16 is a non-portable size: opted in here)
 template <int NT, int CL, bool MIXED>
-static bool launch_group(const STS_Batch b, const BatchParams& prm, const int* order, int count, int* queue, int grid,
-                         cudaStream_t st)
+static bool cluster_fits()
 {
   if constexpr (CL > 8)
-  { // 16-CTA clusters are a non-portable size: opt in, and launch only if one fits
-    static int fits = -1;
-    if (fits < 0)
-    {
-      fits = 0;
+  {
+    static const bool fits = [] {
+      bool ok = false;
       if (cudaFuncSetAttribute(batch_kernel<NT, CL, MIXED>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess)
       {
         cudaLaunchConfig_t q = {};
@@ -623,15 +699,24 @@ static bool launch_group(const STS_Batch b, const BatchParams& prm, const int* o
         q.attrs                = qa;
         q.numAttrs             = 1;
         int nc                 = 0;
-        if (cudaOccupancyMaxActiveClusters(&nc, batch_kernel<NT, CL, MIXED>, &q) == cudaSuccess && nc > 0) fits = 1;
+        ok = cudaOccupancyMaxActiveClusters(&nc, batch_kernel<NT, CL, MIXED>, &q) == cudaSuccess && nc > 0;
       }
       cudaGetLastError();
-    }
-    if (!fits)
-    {
-      sts_set_error("STS_Batch: %d-CTA clusters of %d threads cannot be scheduled", CL, NT);
-      return false;
-    }
+      return ok;
+    }();
+    return fits;
+  }
+  return true;
+}
+
+template <int NT, int CL, bool MIXED>
+static bool launch_group(const STS_Batch b, const BatchParams& prm, const int* order, int count, int* queue, int grid,
+                         cudaStream_t st)
+{
+  if (!cluster_fits<NT, CL, MIXED>())
+  {
+    sts_set_error("STS_Batch: %d-CTA clusters of %d threads cannot be scheduled", CL, NT);
+    return false;
   }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim            = dim3((unsigned)grid, 1, 1);
@@ -673,35 +758,89 @@ static bool launch_cl(const STS_Batch b, const BatchParams& prm, int cl, const i
                    : launch_cl_m<NT, false>(b, prm, cl, order, count, queue, grid, st);
 }
 
-// One launch (cluster size 1), or two concurrent launches: instances with n >= big_n on
-// clusters of `cluster` CTAs (launched first), the rest on single CTAs on a second stream.
-// The CTA slots (SMs x CTAs per SM) are split between the two in proportion to their
-// estimated cost.
+// makes the kernel resident: with lazy loading a first launch beside a running kernel waits for it
+template <int NT, bool MIXED>
+static bool load_cl_m(int cl)
+{
+  cudaFuncAttributes a;
+  const void* f = cl == 16  ? (const void*)batch_kernel<NT, 16, MIXED>
+                  : cl == 8 ? (const void*)batch_kernel<NT, 8, MIXED>
+                  : cl == 4 ? (const void*)batch_kernel<NT, 4, MIXED>
+                  : cl == 2 ? (const void*)batch_kernel<NT, 2, MIXED>
+                            : (const void*)batch_kernel<NT, 1, MIXED>;
+  return STS_CUDA_OK(cudaFuncGetAttributes(&a, f));
+}
+
+template <int NT>
+static bool load_cl(const BatchParams& prm, int cl)
+{
+  return prm.mixed ? load_cl_m<NT, true>(cl) : load_cl_m<NT, false>(cl);
+}
+
+// One launch (cluster size 1), or up to three concurrent ones: the heaviest instances on clusters
+// of 2 x `cluster` CTAs, the others with n >= big_n on clusters of `cluster` CTAs, the rest on
+// single CTAs. The CTA slots (SMs x CTAs per SM) are split in proportion to the estimated cost.
+//
+// A batch ends with its longest instance, and one CTA per SM runs at the FP64 pipe's rate (8
+// instructions per point and stage, 22 at the step end), so an instance's SMs bound it: it is heavy
+// if its cost on `cluster` CTAs exceeds the slots' mean, and gets the next cluster size up to the
+// hardware's 16. 256 instances of 64..512, clusters of 8, device ms: 188-201 one group after the
+// other on 8 CTAs, 203 groups at once, 101 with heavy clusters (twice this limit 100, half 125-143);
+// 64 instances 135, 105, 62-75.
+// Clusters need free slots in one GPC: with every slot taken some wait for a whole instance to
+// end, so a quarter of the slots that fit an SM at once (1024 threads) stays free: 102 ms (median of ten
+// calls) against 132 with all slots, 156 with 7/8, 127 with 5/8. The heavy group has the highest
+// stream priority, so that it is placed first. (Heavy clusters of 1024-thread CTAs with an SM each:
+// 97 to 150 ms, 64 instances 97 against 61.)
 static bool batch_launch(STS_Batch b, const BatchParams& prm, int threads, int ctas_per_sm)
 {
   STS_Context ctx = b->ctx;
   cudaStream_t st = ctx->stream;
-  if (!STS_CUDA_OK(cudaMemsetAsync(b->dqueue, 0, 2 * sizeof(int), st))) return false;
-  const int slots = ctx->num_sms * ctas_per_sm;
+  if (!STS_CUDA_OK(cudaMemsetAsync(b->dqueue, 0, 3 * sizeof(int), st))) return false;
+  const int CL    = b->cluster;
+  const bool split = CL > 1 && b->nbig > 0;
+  const int fit    = ctx->num_sms * (1024 / threads);
+  const int slots  = split ? std::min(ctx->num_sms * ctas_per_sm, fit * 3 / 4) : ctx->num_sms * ctas_per_sm;
+  auto load = [&](int cl) {
+    return threads == 256 ? load_cl<256>(prm, cl) : load_cl<512>(prm, cl);
+  };
   auto go = [&](int cl, const int* order, int count, int* queue, int grid, cudaStream_t s) {
     return threads == 256 ? launch_cl<256>(b, prm, cl, order, count, queue, grid, s)
                           : launch_cl<512>(b, prm, cl, order, count, queue, grid, s);
   };
-  const int CL = b->cluster;
-  if (CL <= 1 || b->nbig == 0)
+  if (!split)
     return go(1, b->dorder, b->ninst, b->dqueue, std::max(1, std::min(b->ninst, slots)), st);
   const int nsmall = b->ninst - b->nbig;
-  int gbig = (int)std::lround(b->big_share * slots / CL) * CL;
-  gbig     = std::max(CL, std::min(gbig, b->nbig * CL));
-  gbig     = std::min(gbig, (slots / CL) * CL);
-  int gsm  = std::max(1, std::min(nsmall, slots - gbig));
-  bool ok  = go(CL, b->dorder_big, b->nbig, b->dqueue, gbig, st);
-  if (ok && nsmall > 0)
-  {
-    ok = STS_CUDA_OK(cudaEventRecord(b->ev_fork, st)) && STS_CUDA_OK(cudaStreamWaitEvent(b->side, b->ev_fork, 0)) &&
-         go(1, b->dorder_small, nsmall, b->dqueue + 1, gsm, b->side) &&
-         STS_CUDA_OK(cudaEventRecord(b->ev_join, b->side)) && STS_CUDA_OK(cudaStreamWaitEvent(st, b->ev_join, 0));
-  }
+  // the heavy instances are the first of the cost-ordered b->order_big
+  int nheavy = 0;
+  if (2 * CL <= 16 && (CL < 8 || (threads == 256 ? (prm.mixed ? cluster_fits<256, 16, true>() : cluster_fits<256, 16, false>())
+                                                 : (prm.mixed ? cluster_fits<512, 16, true>() : cluster_fits<512, 16, false>()))))
+    while (nheavy < b->nbig && b->hinst[b->order_big[nheavy]].n >= 4 * CL &&
+           b->cost[b->order_big[nheavy]] * slots > b->cost_total * CL)
+      ++nheavy;
+  double heavy_share = 0.0;
+  for (int k = 0; k < nheavy; ++k) heavy_share += b->cost[b->order_big[k]] / b->cost_total;
+  auto ctas = [&](double share, int count, int cl, int room) {
+    int g = (int)std::lround(share * slots / cl) * cl;
+    g     = std::max(cl, std::min(g, count * cl));
+    return std::max(cl, std::min(g, room / cl * cl));
+  };
+  const int gheavy = nheavy ? ctas(heavy_share, nheavy, 2 * CL, slots) : 0;
+  const int nbig   = b->nbig - nheavy;
+  const int gbig   = nbig ? ctas(b->big_share - heavy_share, nbig, CL, std::max(CL, slots - gheavy)) : 0;
+  const int gsm    = std::max(1, std::min(nsmall, slots - gheavy - gbig));
+  bool ok          = (!nheavy || load(2 * CL)) && (!nbig || load(CL)) && (!nsmall || load(1)) &&
+            STS_CUDA_OK(cudaEventRecord(b->ev_fork, st));
+  auto beside      = [&](int q, int cl, const int* order, int count, int grid) {
+    return STS_CUDA_OK(cudaStreamWaitEvent(b->side[q], b->ev_fork, 0)) &&
+           go(cl, order, count, b->dqueue + 1 + q, grid, b->side[q]) &&
+           STS_CUDA_OK(cudaEventRecord(b->ev_join[q], b->side[q]));
+  };
+  if (ok && nheavy) ok = beside(0, 2 * CL, b->dorder_big, nheavy, gheavy);
+  if (ok && nbig) ok = beside(1, CL, b->dorder_big + nheavy, nbig, gbig);
+  if (ok && nsmall) ok = go(1, b->dorder_small, nsmall, b->dqueue, gsm, st);
+  if (ok && nheavy) ok = STS_CUDA_OK(cudaStreamWaitEvent(st, b->ev_join[0], 0));
+  if (ok && nbig) ok = STS_CUDA_OK(cudaStreamWaitEvent(st, b->ev_join[1], 0));
   return ok;
 }
 
@@ -722,7 +861,9 @@ static bool batch_regroup(STS_Batch b)
     }
     else small.push_back(i);
   }
-  b->nbig      = (int)big.size();
+  b->nbig       = (int)big.size();
+  b->order_big  = big;
+  b->cost_total = ct;
   b->big_share = ct > 0.0 ? cb / ct : 0.0;
   return (big.empty() || STS_CUDA_OK(cudaMemcpy(b->dorder_big, big.data(), big.size() * sizeof(int),
                                                  cudaMemcpyHostToDevice))) &&
@@ -773,14 +914,18 @@ extern "C" STS_Batch STS_BatchCreate(STS_Context ctx, int ninst, const int* n, c
   std::vector<int> order(ninst);
   std::iota(order.begin(), order.end(), 0);
   std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return cost[x] > cost[y]; });
+  int prio_lo = 0, prio_hi = 0;
+  cudaDeviceGetStreamPriorityRange(&prio_lo, &prio_hi);
   bool ok = STS_CUDA_OK(cudaMalloc(&b->dinst, ninst * sizeof(BatchInst))) &&
             STS_CUDA_OK(cudaMalloc(&b->dorder, ninst * sizeof(int))) &&
             STS_CUDA_OK(cudaMalloc(&b->dorder_big, ninst * sizeof(int))) &&
             STS_CUDA_OK(cudaMalloc(&b->dorder_small, ninst * sizeof(int))) &&
-            STS_CUDA_OK(cudaMalloc(&b->dqueue, 2 * sizeof(int))) &&
-            STS_CUDA_OK(cudaStreamCreateWithFlags(&b->side, cudaStreamNonBlocking)) &&
+            STS_CUDA_OK(cudaMalloc(&b->dqueue, 3 * sizeof(int))) &&
+            STS_CUDA_OK(cudaStreamCreateWithPriority(&b->side[0], cudaStreamNonBlocking, prio_hi)) &&
+            STS_CUDA_OK(cudaStreamCreateWithPriority(&b->side[1], cudaStreamNonBlocking, (prio_hi + prio_lo) / 2)) &&
             STS_CUDA_OK(cudaEventCreateWithFlags(&b->ev_fork, cudaEventDisableTiming)) &&
-            STS_CUDA_OK(cudaEventCreateWithFlags(&b->ev_join, cudaEventDisableTiming)) &&
+            STS_CUDA_OK(cudaEventCreateWithFlags(&b->ev_join[0], cudaEventDisableTiming)) &&
+            STS_CUDA_OK(cudaEventCreateWithFlags(&b->ev_join[1], cudaEventDisableTiming)) &&
             STS_CUDA_OK(cudaMalloc(&b->y, b->total * sizeof(double))) &&
             STS_CUDA_OK(cudaMalloc(&b->work, 6 * b->total * sizeof(double))) &&
             STS_CUDA_OK(cudaMemcpy(b->dinst, b->hinst.data(), ninst * sizeof(BatchInst), cudaMemcpyHostToDevice)) &&
@@ -807,9 +952,11 @@ extern "C" int STS_BatchFree(STS_Batch* pb)
   cudaFree(b->dcoef);
   cudaFree(b->dorder_big);
   cudaFree(b->dorder_small);
-  if (b->side) cudaStreamDestroy(b->side);
+  for (cudaStream_t q : b->side)
+    if (q) cudaStreamDestroy(q);
   if (b->ev_fork) cudaEventDestroy(b->ev_fork);
-  if (b->ev_join) cudaEventDestroy(b->ev_join);
+  for (cudaEvent_t e : b->ev_join)
+    if (e) cudaEventDestroy(e);
   delete b;
   *pb = nullptr;
   return 0;

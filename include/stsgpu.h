@@ -476,7 +476,8 @@ int STS_BatchAutotune(STS_Batch b, double tf_probe, int method, double rtol, dou
 /* instances with n >= big_n are integrated by thread-block clusters of `cluster` CTAs (1, 2,
  * 4, 8, or 16 where the device schedules that non-portable size; rows split between the
  * CTAs, cluster barriers between sweeps, the exact reductions combined through distributed
- * shared memory), concurrently with the single-CTA group */
+ * shared memory), concurrently with the single-CTA group. An instance whose estimated cost on that
+ * many CTAs exceeds the mean of the CTA slots gets twice as many (up to 16); results are the same. */
 int STS_BatchSetCluster(STS_Batch b, int cluster, int big_n);
 int STS_BatchGetLaunch(STS_Batch b, int* threads, int* ctas_per_sm, int* cluster, int* big_n);
 

@@ -123,3 +123,22 @@ def test_batch_autotune_keeps_results(ctx, stslib):
     C.set_launch(th, cp)
     C.evolve(0.005)
     assert np.array_equal(B.state(), C.state())
+
+
+@pytest.mark.parametrize("mixed", [False, True])
+@pytest.mark.parametrize("cluster", [2, 4, 8])
+@pytest.mark.parametrize("off", [-1, 0, 1])
+def test_batch_heavy_instances_agree_bitwise(ctx, stslib, mixed, cluster, off):
+    """The heaviest instances run on twice the cluster from n = 4 x cluster on: sizes around that
+    line and ragged rows per CTA, beside instances of the other two groups, equal single CTAs."""
+    rng = np.random.default_rng(cluster)
+    inst = [(n, 1.0, 0.5, np.array([1, 3]), np.array([2, 1]), rng.standard_normal(2))
+            for n in (4 * cluster + off, 67, 33, 40, 5, 12)]
+    out = []
+    for shape in ((256, 1, 1), (256, 4, cluster), (512, 1, cluster)):
+        B = stslib.Batch(ctx, inst)
+        assert B.set_mixed(mixed) in (None, 0)
+        B.set_launch(*shape, big_n=min(33, 4 * cluster + off))
+        B.evolve(0.01, method=stslib.RKC, rtol=1e-6, atol=1e-10)
+        out.append(B.state())
+    assert np.array_equal(out[0], out[1]) and np.array_equal(out[0], out[2])
