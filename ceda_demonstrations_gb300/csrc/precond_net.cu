@@ -27,6 +27,7 @@
 #include <random>
 #include <vector>
 
+#include "soft64.cuh"
 #include "sts_internal.cuh"
 
 namespace net {
@@ -631,7 +632,7 @@ __device__ __forceinline__ void convert_row(const unsigned char* raw, unsigned c
 
 // MODE 0: BF16 NHWC output (POOL: also the 2x2 means of the round's row pair into pout, in the
 // order of pool_kernel); MODE 2: z = (out_scale scale) r + (double)((float)out_scale u),
-// u = c0 + sk c1 + sg c2, as conv_epilogue. wu: the nine taps' B operands (tc_weight_kernel).
+// u = c0 + sk c1 + sg c2, as conv_epilogue. wu: the nine taps' B operands (tc_weight).
 // Segments start on even rows and H is even, so every round has two rows.
 template <int MODE, int LOAD, bool POOL>
 __global__ void __launch_bounds__(tc::COLS) conv3x3_tc_kernel(const __nv_bfloat16* __restrict__ in, int H, int W,
@@ -1106,12 +1107,10 @@ __global__ void __launch_bounds__(ZTX * ZTY) z_kernel(const double* __restrict__
 
 // The nine taps' B operands (B[n = output channel][k = input channel], K-major without
 // swizzle: byte t*512 + (n/8)*256 + (k/8)*128 + (n%8)*16 + (k%8)*2) of a layer, forward or
-// transposed (swapped channels, flipped taps), as frag_kernel's weights
-__global__ void tc_weight_kernel(const float* __restrict__ W, __nv_bfloat16* __restrict__ wu, int transpose)
+// transposed (swapped channels, flipped taps), as frag_weight's weights
+__device__ __forceinline__ void tc_weight(const float* __restrict__ W, __nv_bfloat16* __restrict__ wu, int transpose, int e)
 {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x; // 0 .. 9*256
-  if (e >= 9 * 256) return;
-  const int t = e >> 8, n = (e >> 4) & 15, k = e & 15;
+  const int t = e >> 8, n = (e >> 4) & 15, k = e & 15; // e: 0 .. 9*256
   const float v = transpose ? W[(k * CH + n) * 9 + (8 - t)] : W[(n * CH + k) * 9 + t];
   wu[t * 256 + (n >> 3) * 128 + (k >> 3) * 64 + (n & 7) * 8 + (k & 7)] = __float2bfloat16_rn(v);
 }
@@ -1206,39 +1205,51 @@ __global__ void poolT_add_kernel(const __nv_bfloat16* __restrict__ gcoarse, int 
 // Energy-norm loss of each image (n x n): d = z - e, L_img = 0.5 d^T M d / (e^T M e) with
 // M = I - gamma A on the crop (zero outside). With g = (M d) * out_scale / (e^T M e) * gscale
 // the gradient of the last transposed convolution's output channels is [g, sk g, sg g] (BF16);
-// adds gscale * sum L_img to *acc.
-__global__ void gradz_kernel(long long npix, int n, const double* __restrict__ z, const float* __restrict__ e,
-                             double gscale, const float* __restrict__ meta, __nv_bfloat16* __restrict__ g,
-                             double* __restrict__ acc)
+// adds gscale * sum L_img to *acc. Bound by the FP64 pipe: a thread marches GZ_ROWS rows of one
+// image's column, the image's factors (a division) formed once per thread and z - e of the column
+// once per point: 32 images of 128^2 52 -> 32 us (2, 4 and 8 rows alike).
+constexpr int GZ_ROWS = 4;
+__global__ void __launch_bounds__(256) gradz_kernel(int n, int nimg, const double* __restrict__ z,
+                                                   const float* __restrict__ e, double gscale,
+                                                   const float* __restrict__ meta, __nv_bfloat16* __restrict__ g,
+                                                   double* __restrict__ acc)
 {
-  const long long ip = (long long)n * n;
-  double lsum        = 0.0;
-  for (long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x; p < npix; p += (long long)gridDim.x * blockDim.x)
+  const int i  = blockIdx.x * 32 + threadIdx.x;
+  const int jb = (blockIdx.y * 8 + threadIdx.y) * GZ_ROWS, je = min(jb + GZ_ROWS, n);
+  double lsum  = 0.0;
+  for (int img = blockIdx.z; img < nimg; img += gridDim.z)
   {
-    const int img = (int)(p / ip);
-    const int q = (int)(p % ip), i = q % n, j = q / n;
-    const float* m = meta + META * img;
-    const double gcx = m[5], gcy = m[6];
-    auto dd = [&](long long k) { return z[k] - (double)e[k]; };
-    const double dc = dd(p);
-    const double dw = i > 0 ? dd(p - 1) : 0.0, de = i < n - 1 ? dd(p + 1) : 0.0;
-    const double ds = j > 0 ? dd(p - n) : 0.0, dn = j < n - 1 ? dd(p + n) : 0.0;
-    const double Md = (1.0 + 2.0 * (gcx + gcy)) * dc - gcx * (dw + de) - gcy * (ds + dn);
-    const double inv = (double)m[4];
-    lsum += 0.5 * dc * Md * inv;
-    const float gv = (float)(Md * inv * meta_out_scale(meta, img) * gscale);
-    __align__(16) __nv_bfloat16 o[CH];
-    o[0] = __float2bfloat16_rn(gv); // dL/du expanded over the input channels [1, sk, sg]
-    o[1] = __float2bfloat16_rn(gv * m[0]);
-    o[2] = __float2bfloat16_rn(gv * m[1]);
+    if (i >= n || jb >= n) break;
+    const float* m   = meta + META * img;
+    const double gcx = m[5], gcy = m[6], d = 1.0 + 2.0 * (gcx + gcy), inv = (double)m[4];
+    const double os  = meta_out_scale(meta, img);
+    const float m0 = m[0], m1 = m[1];
+    long long p = ((long long)img * n + jb) * n + i;
+    auto dd     = [&](long long k) { return z[k] - s64_from_float(e[k]); };
+    double ds = jb > 0 ? dd(p - n) : 0.0, dc = dd(p);
+#pragma unroll 2
+    for (int j = jb; j < je; ++j, p += n)
+    {
+      const double dw = i > 0 ? dd(p - 1) : 0.0, de = i < n - 1 ? dd(p + 1) : 0.0;
+      const double dn = j < n - 1 ? dd(p + n) : 0.0;
+      const double Md = d * dc - gcx * (dw + de) - gcy * (ds + dn);
+      lsum += 0.5 * dc * Md * inv;
+      const float gv = (float)(Md * inv * os * gscale);
+      __align__(16) __nv_bfloat16 o[CH];
+      o[0] = __float2bfloat16_rn(gv); // dL/du expanded over the input channels [1, sk, sg]
+      o[1] = __float2bfloat16_rn(gv * m0);
+      o[2] = __float2bfloat16_rn(gv * m1);
 #pragma unroll
-    for (int c = 3; c < CH; ++c) o[c] = __float2bfloat16_rn(0.f);
-    uint4* dst = reinterpret_cast<uint4*>(g + p * CH);
-    dst[0]     = reinterpret_cast<uint4*>(o)[0];
-    dst[1]     = reinterpret_cast<uint4*>(o)[1];
+      for (int c = 3; c < CH; ++c) o[c] = __float2bfloat16_rn(0.f);
+      uint4* dst = reinterpret_cast<uint4*>(g + p * CH);
+      dst[0]     = reinterpret_cast<uint4*>(o)[0];
+      dst[1]     = reinterpret_cast<uint4*>(o)[1];
+      ds         = dc;
+      dc         = dn;
+    }
   }
   for (int m = 16; m >= 1; m >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, m);
-  if ((threadIdx.x & 31) == 0 && lsum != 0.0) atomicAdd(acc, lsum * gscale);
+  if (threadIdx.x == 0 && lsum != 0.0) atomicAdd(acc, lsum * gscale);
 }
 
 // per-pair metadata from the harvested crops: scale = 1/rms(r), 1/(e^T M e); one block per pair
@@ -1450,10 +1461,8 @@ namespace net {
 
 // fragment layout of one layer's weights (BF16, see conv3x3_march_kernel); transpose = 1 builds
 // the input-gradient weights W'[ci][co][8 - t] = W[co][ci][t]
-__global__ void frag_kernel(const float* __restrict__ W, uint2* __restrict__ wf, int transpose)
-{
-  const int k = blockIdx.x * blockDim.x + threadIdx.x; // 0 .. 9*2*32
-  if (k >= 9 * 2 * 32) return;
+__device__ __forceinline__ void frag_weight(const float* __restrict__ W, uint2* __restrict__ wf, int transpose, int k)
+{ // k: 0 .. 9*2*32
   const int lane = k & 31, nh = (k >> 5) & 1, t = k >> 6;
   const int co = nh * 8 + (lane >> 2), ci0 = (lane & 3) * 2;
   auto w = [&](int o, int i) -> float {
@@ -1465,6 +1474,22 @@ __global__ void frag_kernel(const float* __restrict__ W, uint2* __restrict__ wf,
   v.x   = *reinterpret_cast<uint32_t*>(&lo);
   v.y   = *reinterpret_cast<uint32_t*>(&hi);
   wf[k] = v;
+}
+
+// all layouts of all layers' weights in one launch (16 launches cost 45 us of a 430 us minibatch):
+// grid.y the layer; of 24 blocks 3 + 3 write the MMA fragments, 9 + 9 the tcgen05 operands
+__global__ void __launch_bounds__(256) weight_layouts_kernel(const float* __restrict__ w, uint2* __restrict__ wf,
+                                                            uint2* __restrict__ wt, __nv_bfloat16* __restrict__ wu,
+                                                            __nv_bfloat16* __restrict__ wut)
+{
+  const int l = blockIdx.y, b = blockIdx.x;
+  const float* W = w + l * WSZ;
+  if (b < 6)
+  {
+    const int k = (b % 3) * 256 + threadIdx.x;
+    if (k < 576) frag_weight(W, (b < 3 ? wf : wt) + l * 576, b >= 3, k);
+  }
+  else tc_weight(W, (b < 15 ? wu : wut) + l * 9 * 256, b >= 15, ((b - 6) % 9) * 256 + threadIdx.x);
 }
 
 // x = [r, r sk, r sg] * scale (BF16 NHWC, channels 3..15 zero); with meta, sk, sg and scale
@@ -1622,14 +1647,7 @@ static bool ensure_capacity(STS_Net nt, long long pix)
 
 static void refresh_frags(STS_Net nt)
 {
-  cudaStream_t st = nt->ctx->stream;
-  for (int l = 0; l < NLAYER; ++l)
-  {
-    net::frag_kernel<<<3, 256, 0, st>>>(nt->w + l * WSZ, nt->wf + l * 576, 0);
-    net::frag_kernel<<<3, 256, 0, st>>>(nt->w + l * WSZ, nt->wt + l * 576, 1);
-    net::tc_weight_kernel<<<9, 256, 0, st>>>(nt->w + l * WSZ, nt->wu + l * 9 * 256, 0);
-    net::tc_weight_kernel<<<9, 256, 0, st>>>(nt->w + l * WSZ, nt->wut + l * 9 * 256, 1);
-  }
+  net::weight_layouts_kernel<<<dim3(24, NLAYER), 256, 0, nt->ctx->stream>>>(nt->w, nt->wf, nt->wt, nt->wu, nt->wut);
   nt->win_stale = true;
 }
 
@@ -2063,10 +2081,11 @@ static void net_backward(STS_Net nt, int n, int nimg, const float* e, double gsc
 {
   cudaStream_t st = nt->ctx->stream;
   net::Level* L   = nt->L;
-  const long long ip = (long long)n * n, np = ip * nimg;
   const int m = nimg;
   net::WgradParts q;
-  net::gradz_kernel<<<grid_for(np), 256, 0, st>>>(np, n, nt->z, e, gscale, meta, L[0].dy, nt->dacc); // d gx (3 ch)
+  const int gz = 8 * net::GZ_ROWS;
+  const dim3 gg((n + 31) / 32, (n + gz - 1) / gz, (unsigned)std::min(m, 65535));
+  net::gradz_kernel<<<gg, dim3(32, 8), 0, st>>>(n, m, nt->z, e, gscale, meta, L[0].dy, nt->dacc); // d gx (3 ch)
   // adjoint pass, top (level 0) to bottom (level 3)
   wgrad(nt, q, 0, L[0].dy, L[0].g, n, m, net::L_IN);                 // W_in via convT(g0)
   conv(nt, L[0].dy, n, m, net::L_IN, false, L[0].dg);          // d g0 (= d h0 so far)
