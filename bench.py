@@ -158,18 +158,24 @@ def mixed_stage_traffic(n):
 #       python bench.py --n 6144 --steps 1 --warmup 3 --no-cpu --stage-fusion 4 --fusion-config 2
 # 6144^2: 459.5 MB read + 260.0 MB written = 719.5 MB per launch (algorithmic 754.9 MB).
 TRAFFIC_FUSED4_6144 = 719.5e6
+# The eight-stage kernel (112 x 48 tiles) the same way, autotuned (no --stage-fusion, -s 30):
+# 476.9 MB read + 265.1 MB written.
+TRAFFIC_FUSED8_6144 = 742.0e6
 
 
-def fused_stage_traffic(n):
-    return TRAFFIC_FUSED4_6144 * (n / 6144.0) ** 2
+def fused_stage_traffic(n, ks=4):
+    return (TRAFFIC_FUSED8_6144 if ks == 8 else TRAFFIC_FUSED4_6144) * (n / 6144.0) ** 2
 
 
 def step_launches(stages, ks):
     """Kernels one step attempt of `stages` stages launches on the fused mixed path: stage 1,
     the stages 2..s one per launch (ks = 1) or in groups of ks with a shorter last group (a
-    last group of one stage runs as a single-stage launch), and the step end."""
+    last group of one stage runs as a single-stage launch), and the step end. Groups of eight are
+    followed by groups of four for the seven stages or fewer that remain."""
     if ks <= 1:
         return stages + 1
+    if ks == 8:
+        return 2 + (stages - 1) // 8 + ((stages - 1) % 8 + 3) // 4
     return 2 + (stages - 2 + ks) // ks
 
 
@@ -355,10 +361,11 @@ def run_gpu(args):
     stage_bytes_mixed = (20.0 if ks > 1 else 16.0) * N2
     stage_bytes_fp64 = 40.0 * N2
     ach = stage_bytes_mixed / (m["stage_ms"] / 1e3) / 1e9
-    traffic = fused_stage_traffic(n) if ks > 1 else mixed_stage_traffic(n)
+    traffic = fused_stage_traffic(n, ks) if ks > 1 else mixed_stage_traffic(n)
     if ks > 1:
-        kdesc = ("mixed stages, %d per launch on 120x%d shared-memory tiles (20 B per point and launch, "
-                 "%.1f B/DOF-stage): %s" % (ks, m["kinfo"]["fusion"]["tile_rows"], 20.0 / ks, m["kinfo"]["name"]))
+        kdesc = ("mixed stages, %d per launch on %dx%d shared-memory tiles (20 B per point and launch, "
+                 "%.1f B/DOF-stage; bound by instruction issue): %s" % (ks, 112 if ks == 8 else 120, m["kinfo"]["fusion"]["tile_rows"], 20.0 / ks,
+                                            m["kinfo"]["name"]))
     else:
         kdesc = "mixed stage kernel (16 B/DOF-stage), autotuned: %s" % m["kinfo"]["name"]
     fp64_flops = 17.0 * N2 / (d["stage_ms"] / 1e3)
@@ -404,7 +411,8 @@ def run_gpu(args):
                  "fp64_peak_tflops_probed": fp64_peak_tflops,
                  "stage_kernel_fp64_frac": (fp64_flops / 1e12 / fp64_peak_tflops) if fp64_peak_tflops else None,
                  "fp64_peak_note": "FP64 FMA rate probed in this run (STS_ProbeFP64Rate: independent FMA "
-                                   "chains, 8 blocks per SM); the stage kernel does 17 flops per DOF-stage"},
+                                   "chains, 8 blocks per SM); the stage kernel does 17 flops per DOF-stage, part "
+                                   "of them as integer code with the same bits, so the fraction may exceed 1"},
         "speedup_mixed_vs_fp64": value / fp64_value,
         "accuracy": {"t": m["t"], "mixed_rel_l2_vs_exact": out[True], "fp64_rel_l2_vs_exact": out[False],
                      "mixed_vs_fp64_rel_l2": mix_vs_64},

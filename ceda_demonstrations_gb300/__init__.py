@@ -624,7 +624,7 @@ class LSRKStep:
 
     def stage_fusion_info(self):
         """Stages per launch in use (1: one launch per stage), the tile configuration (0: none)
-        and its rows, and the autotuner's milliseconds per four-stage launch."""
+        and its rows, and the autotuner's milliseconds per launch of a group."""
         ks, cfg, rows, ms = C.c_int(), C.c_int(), C.c_int(), C.c_double()
         lib().STS_LSRKStepGetStageFusion(self.mem, C.byref(ks), C.byref(cfg), C.byref(rows), C.byref(ms))
         return {"ks": ks.value, "config": cfg.value, "tile_rows": rows.value, "ms": ms.value}

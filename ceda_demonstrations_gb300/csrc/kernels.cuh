@@ -138,24 +138,6 @@ __device__ __forceinline__ double mixed_weight(double rtol, double atol, double 
 template <typename T, int V>
 struct VecIO;
 template <>
-struct VecIO<double, 1> {
-  static __device__ __forceinline__ void ld(const double* p, double (&v)[1]) { v[0] = __ldg(p); }
-  static __device__ __forceinline__ void st(double* p, const double (&v)[1]) { p[0] = v[0]; }
-};
-template <>
-struct VecIO<double, 2> {
-  static __device__ __forceinline__ void ld(const double* p, double (&v)[2])
-  {
-    double2 t = __ldg(reinterpret_cast<const double2*>(p));
-    v[0]      = t.x;
-    v[1]      = t.y;
-  }
-  static __device__ __forceinline__ void st(double* p, const double (&v)[2])
-  {
-    *reinterpret_cast<double2*>(p) = make_double2(v[0], v[1]);
-  }
-};
-template <>
 struct VecIO<float, 1> {
   static __device__ __forceinline__ void ld(const float* p, float (&v)[1]) { v[0] = __ldg(p); }
   static __device__ __forceinline__ void st(float* p, const float (&v)[1]) { p[0] = v[0]; }

@@ -26,3 +26,14 @@ def test_step_launches_follow_the_stage_schedule(ks):
         want = s + 1 if ks == 1 else schedule(s, ks)
         assert bench.step_launches(s, ks) == want, (s, ks)
     assert bench.step_launches(196, 4) == 51  # the 8192^2 workload's steps
+
+
+def test_step_launches_with_groups_of_eight():
+    """Groups of eight while eight stages remain, then groups of four, a last single stage alone."""
+    for s in range(2, 201):
+        launches, j = 2, 2
+        while j <= s:
+            left = s - j + 1
+            j += 8 if left >= 8 else min(4, left)
+            launches += 1
+        assert bench.step_launches(s, 8) == launches, s
