@@ -784,14 +784,14 @@ static bool load_cl(const BatchParams& prm, int cl)
 // A batch ends with its longest instance, and one CTA per SM runs at the FP64 pipe's rate (8
 // instructions per point and stage, 22 at the step end), so an instance's SMs bound it: it is heavy
 // if its cost on `cluster` CTAs exceeds the slots' mean, and gets the next cluster size up to the
-// hardware's 16. 256 instances of 64..512, clusters of 8, device ms: 188-201 one group after the
-// other on 8 CTAs, 203 groups at once, 101 with heavy clusters (twice this limit 100, half 125-143);
-// 64 instances 135, 105, 62-75.
-// Clusters need free slots in one GPC: with every slot taken some wait for a whole instance to
-// end, so a quarter of the slots that fit an SM at once (1024 threads) stays free: 102 ms (median of ten
-// calls) against 132 with all slots, 156 with 7/8, 127 with 5/8. The heavy group has the highest
-// stream priority, so that it is placed first. (Heavy clusters of 1024-thread CTAs with an SM each:
-// 97 to 150 ms, 64 instances 97 against 61.)
+// hardware's 16. Clusters need free slots in one GPC: with every slot theirs some wait for a whole
+// instance to end, so they share three quarters of the slots that fit an SM at once (1024 threads):
+// 102 ms (median of ten calls) against 132 with all, 156 with 7/8, 127 with 5/8. The single CTAs,
+// launched last and with the lowest stream priority, take what is left, since the estimate is low for small
+// instances. Device ms for four draws of 256 instances of 64..512, clusters of 8: one group after the
+// other 196 179 210 203, with heavy clusters and the groups side by side 104 113 174 184, singles in
+// the free slots 105 109 128 123; two draws of 64 instances 136 142, now 61 80. (Twice the limit for
+// heavy or half of it is no better; heavy clusters of 1024-thread CTAs with an SM each 97 to 166.)
 static bool batch_launch(STS_Batch b, const BatchParams& prm, int threads, int ctas_per_sm)
 {
   STS_Context ctx = b->ctx;
@@ -828,7 +828,7 @@ static bool batch_launch(STS_Batch b, const BatchParams& prm, int threads, int c
   const int gheavy = nheavy ? ctas(heavy_share, nheavy, 2 * CL, slots) : 0;
   const int nbig   = b->nbig - nheavy;
   const int gbig   = nbig ? ctas(b->big_share - heavy_share, nbig, CL, std::max(CL, slots - gheavy)) : 0;
-  const int gsm    = std::max(1, std::min(nsmall, slots - gheavy - gbig));
+  const int gsm    = std::max(1, std::min(nsmall, std::min(ctx->num_sms * ctas_per_sm, fit) - gheavy - gbig));
   bool ok          = (!nheavy || load(2 * CL)) && (!nbig || load(CL)) && (!nsmall || load(1)) &&
             STS_CUDA_OK(cudaEventRecord(b->ev_fork, st));
   auto beside      = [&](int q, int cl, const int* order, int count, int grid) {
