@@ -2452,6 +2452,7 @@ __global__ void __launch_bounds__(256) fcg_q_kernel(ProbDev P, const double* __r
   if (s->state != 0) return;
   const double gamma = s->gamma;
   const double c0 = 1.0 - gamma * P.cc, c1 = -gamma * P.cx, c2 = -gamma * P.cy;
+  const soft64::Factor c0F = soft64::factor(c0);
   xsum::Limbs a[1];
   unsigned fl[1] = {0};
   xsum::zero(a[0]);
@@ -2467,7 +2468,9 @@ __global__ void __launch_bounds__(256) fcg_q_kernel(ProbDev P, const double* __r
       const double ps   = (j > 0) ? p[k - nx] : 0.0;
       const double pn   = (j < ny - 1) ? p[k + nx] : 0.0;
       const double sx = pw + pe, sy = ps + pn;
-      const double qk = __fma_rn(c1, sx, __fma_rn(c2, sy, c0 * pc));
+      // (this product as integer code: 24 iterations at 2048^2 7.71 -> 7.50 ms; the dot product's
+      // too 7.77, the integer side is then the fuller one)
+      const double qk = __fma_rn(c1, sx, __fma_rn(c2, sy, s64_mul(c0F, c0, pc)));
       q[k]            = qk;
       xsum::add(a[0], pc * qk, fl[0]);
     }
