@@ -171,9 +171,9 @@ struct VecIO<float, 4> {
 // are no faster (62.6 against 62.0 us at 2048^2) and slower on small grids; with 8 rows five
 // blocks per SM (219 us at 4096^2; four 227, six 222, three 251), else four.
 // Small grids are bound by the latency of the rows that one thread takes in turn (about 1 us
-// each): see launch_stage64 for the rows per thread.
+// each), and there the FP64 instructions (SOFT false) are the shorter chain: see launch_stage64.
 // ---------------------------------------------------------------------------------------
-template <int RY, bool FORCED>
+template <int RY, bool FORCED, bool SOFT>
 __global__ void __launch_bounds__(256, RY == 8 ? 5 : 4) stage64_kernel(ProbDev P, const StageArgs* __restrict__ A,
                                                          const double* __restrict__ ym1,
                                                          const double* __restrict__ ym2,
@@ -205,13 +205,13 @@ __global__ void __launch_bounds__(256, RY == 8 ? 5 : 4) stage64_kernel(ProbDev P
     const double w  = (i > 0) ? __ldg(ym1 + k - 1) : 0.0;
     const double e  = (i + 1 < nx) ? __ldg(ym1 + k + 1) : 0.0;
     const double m2 = __ldg(ym2 + k), z0 = __ldg(y0 + k), q0 = __ldg(f0 + k);
-    const double sx = s64_add(w, e), sy = s64_add(up, dn);
-    double acc      = s64_mul(gcF, gc, cur);
+    const double sx = s64_add<SOFT>(w, e), sy = s64_add<SOFT>(up, dn);
+    double acc      = s64_mul<SOFT>(gcF, gc, cur);
     acc             = __fma_rn(gx, sx, acc);
     acc             = __fma_rn(gy, sy, acc);
     acc             = __fma_rn(gn, m2, acc);
     acc             = __fma_rn(g0, z0, acc);
-    acc             = s64_fma_small(gfF, gf, q0, acc);
+    acc             = s64_fma_small<SOFT>(gfF, gf, q0, acc);
     if (FORCED)
     {
       acc = __fma_rn(__ldg(P.Sy + j), Pi, acc);

@@ -628,24 +628,28 @@ static void dispatch_forced(bool forced, F&& f)
 // blocks of 256 per SM), then 2, 4 and 8 rows as the grid gets waves to spare. Measured us per
 // stage with 1 / 2 / 4 / 8 rows: 128^2 3.3 / 4.1 / 5.8 / 9.0, 384^2 5.16 / 5.12 / 6.1 / 9.8,
 // 512^2 7.2 / 7.2 / 7.4 / 9.5, 1024^2 20.3 / 18.2 / 17.7 / 19.3, 2048^2 82 / 70 / 63.5 / 62.0.
+// Below half of W the FP64 pipe is not the bound and the integer forms only lengthen the chain:
+// 128^2 2.77 us with them, 2.41 without; 300 x 200 3.2 either way; 384^2 4.2 with, 4.9 without.
 static void launch_stage64(LSRKMem* m, STS_Problem p, const StageArgs* A, const double* ym1, const double* ym2,
                            const double* y0, const double* f0, double* yj)
 {
   const bool forced = p->kind == STS_PROBLEM_MANUFACTURED;
   dim3 b(64, 4);
-  auto go = [&](auto Rc) {
+  auto go = [&](auto Rc, auto Sc) {
     constexpr int R = decltype(Rc)::value;
     dim3 g((unsigned)((p->nx + b.x - 1) / b.x), (unsigned)((p->ny + b.y * R - 1) / (b.y * R)));
     dispatch_forced(forced, [&](auto F) {
-      stage64_kernel<R, decltype(F)::value><<<g, b, 0, m->ctx->stream>>>(p->dev, A, ym1, ym2, y0, f0, yj);
+      stage64_kernel<R, decltype(F)::value, decltype(Sc)::value>
+        <<<g, b, 0, m->ctx->stream>>>(p->dev, A, ym1, ym2, y0, f0, yj);
     });
   };
   const long long n = p->nx * p->ny, W = 1024LL * m->ctx->num_sms;
   const long long nyb = p->ny / (4 * 65535); // the grid's second dimension ends at 65535 blocks
-  if (n < W && nyb < 1) go(std::integral_constant<int, 1>{});
-  else if (n < 3 * W && nyb < 2) go(std::integral_constant<int, 2>{});
-  else if (n < 10 * W && nyb < 4) go(std::integral_constant<int, 4>{});
-  else go(std::integral_constant<int, 8>{});
+  if (2 * n < W && nyb < 1) go(std::integral_constant<int, 1>{}, std::false_type{});
+  else if (n < W && nyb < 1) go(std::integral_constant<int, 1>{}, std::true_type{});
+  else if (n < 3 * W && nyb < 2) go(std::integral_constant<int, 2>{}, std::true_type{});
+  else if (n < 10 * W && nyb < 4) go(std::integral_constant<int, 4>{}, std::true_type{});
+  else go(std::integral_constant<int, 8>{}, std::true_type{});
 }
 
 static void launch_stage32(LSRKMem* m, STS_Problem p, const StageArgs* A, const float* dm1, const float* dm2,
@@ -1373,19 +1377,20 @@ __device__ __forceinline__ PeriodicColumn periodic_column(const ProbDev& P, long
 }
 
 // periodic_point's operations on values at hand
+template <bool SOFT>
 __device__ __forceinline__ double periodic_value(const PeriodicColumn& c, double s, double n, double uC, double uW,
                                                  double uE, double uS, double uN)
 {
-  double v = s64_mul(-s64_add(c.sum, s64_add(s, n)), uC);
-  v        = __dadd_rn(v, s64_mul(c.wF, c.w, uW));
-  v        = __dadd_rn(v, s64_mul(c.eF, c.e, uE));
-  v        = __dadd_rn(v, s64_mul(s, uS));
-  v        = __dadd_rn(v, s64_mul(n, uN));
+  double v = s64_mul<SOFT>(-s64_add<SOFT>(c.sum, s64_add<SOFT>(s, n)), uC);
+  v        = __dadd_rn(v, s64_mul<SOFT>(c.wF, c.w, uW));
+  v        = __dadd_rn(v, s64_mul<SOFT>(c.eF, c.e, uE));
+  v        = __dadd_rn(v, s64_mul<SOFT>(s, uS));
+  v        = __dadd_rn(v, s64_mul<SOFT>(n, uN));
   return v;
 }
 
 // f(i, j, k, value of the operator on u) for the rows of this thread
-template <int RY, typename F>
+template <int RY, bool SOFT, typename F>
 __device__ __forceinline__ void periodic_march(const ProbDev& P, const double* __restrict__ u, F f)
 {
   const long long nx = P.nx, ny = P.ny;
@@ -1401,13 +1406,13 @@ __device__ __forceinline__ void periodic_march(const ProbDev& P, const double* _
   {
     const double dn = u[(j == ny - 1 ? 0 : j + 1) * nx + i];
     const long long k = j * nx + i;
-    f(k, cur, periodic_value(c, __ldg(P.Dys + j), __ldg(P.Dyn + j), cur, u[j * nx + iw], u[j * nx + ie], up, dn));
+    f(k, cur, periodic_value<SOFT>(c, __ldg(P.Dys + j), __ldg(P.Dyn + j), cur, u[j * nx + iw], u[j * nx + ie], up, dn));
     up  = cur;
     cur = dn;
   }
 }
 
-template <int RY>
+template <int RY, bool SOFT>
 __global__ void __launch_bounds__(256) periodic_stage_kernel(ProbDev P, double c0, double c1, double c2, double c3,
                                                              double c4, const double* __restrict__ ym1,
                                                              const double* __restrict__ ym2,
@@ -1415,8 +1420,8 @@ __global__ void __launch_bounds__(256) periodic_stage_kernel(ProbDev P, double c
                                                              const double* __restrict__ f0, double* __restrict__ yj)
 {
   const soft64::Factor c0F = soft64::factor(c0);
-  periodic_march<RY>(P, ym1, [&](long long k, double u, double fj) {
-    double acc = s64_mul(c0F, c0, u);
+  periodic_march<RY, SOFT>(P, ym1, [&](long long k, double u, double fj) {
+    double acc = s64_mul<SOFT>(c0F, c0, u);
     acc        = __fma_rn(c1, ym2[k], acc);
     acc        = __fma_rn(c2, y0[k], acc);
     acc        = __fma_rn(c3, fj, acc);
@@ -1437,7 +1442,7 @@ __global__ void __launch_bounds__(256) periodic_end_kernel(ProbDev P, const doub
   xsum::zero(acc);
   unsigned flags = 0;
   const soft64::Factor c8F = soft64::factor(0.8), rtF = soft64::factor(rtol);
-  periodic_march<RY>(P, ys, [&](long long k, double u, double f) {
+  periodic_march<RY, true>(P, ys, [&](long long k, double u, double f) {
     fs[k]           = f;
     const double yv = y[k];
     double e        = s64_mul(c8F, 0.8, yv);
@@ -1451,22 +1456,25 @@ __global__ void __launch_bounds__(256) periodic_end_kernel(ProbDev P, const doub
   xsum_block_finish<256>(acc, flags, w, slot, 1, (double)(P.nx * P.ny));
 }
 
-// launch of a kernel that marches rows of a periodic problem: g(rows per thread, grid, block).
+// launch of a kernel that marches rows of a periodic problem: g(rows per thread, integer products
+// or not, grid, block).
 // Measured us per stage with 1 / 2 / 4 / 8 rows (W: the resident threads, 1024 per SM): 128^2 5.1 /
-// 6.1 / - / 14.4, 1000 x 768 (5 W) 22.7 / 22.6 / 24.6 / 24.7, 2048^2 (27 W) 104 / 96 / 97 / 97.
+// 6.1 / - / 14.4, 1000 x 768 (5 W) 22.7 / 22.6 / 24.6 / 24.7, 2048^2 (27 W) 104 / 96 / 97 / 97; 198 x
+// 147 with FP64 products 4.2 against 5.4, 384^2 8.2 either way (as in launch_stage64).
 template <typename G>
 static void periodic_rows(STS_Context ctx, STS_Problem p, G&& g)
 {
   const long long n = p->nx * p->ny, W = 1024LL * ctx->num_sms;
   const long long nyb = p->ny / (4 * 65535); // the grid's second dimension ends at 65535 blocks
-  auto go = [&](auto Rc) {
+  auto go = [&](auto Rc, auto Sc) {
     constexpr int R = decltype(Rc)::value;
     const dim3 b(64, 4);
-    g(Rc, dim3((unsigned)((p->nx + b.x - 1) / b.x), (unsigned)((p->ny + b.y * R - 1) / (b.y * R))), b);
+    g(Rc, Sc, dim3((unsigned)((p->nx + b.x - 1) / b.x), (unsigned)((p->ny + b.y * R - 1) / (b.y * R))), b);
   };
-  if (n < W && nyb < 1) go(std::integral_constant<int, 1>{});
-  else if (n < 10 * W && nyb < 2) go(std::integral_constant<int, 2>{});
-  else go(std::integral_constant<int, 8>{});
+  if (2 * n < W && nyb < 1) go(std::integral_constant<int, 1>{}, std::false_type{});
+  else if (n < W && nyb < 1) go(std::integral_constant<int, 1>{}, std::true_type{});
+  else if (n < 10 * W && nyb < 2) go(std::integral_constant<int, 2>{}, std::true_type{});
+  else go(std::integral_constant<int, 8>{}, std::true_type{});
 }
 
 // Mixed reference mode: FP32 increments d_j = Y_j - Y_0 of the periodic problem in the
@@ -1678,8 +1686,8 @@ static int evolve_generic(LSRKMem* m, double tout, double clip, int itask)
         if (pf)
         {
           STS_Problem p = (STS_Problem)m->user_data;
-          periodic_rows(m->ctx, p, [&](auto R, dim3 g, dim3 b) {
-            periodic_stage_kernel<decltype(R)::value><<<g, b, 0, m->ctx->stream>>>(
+          periodic_rows(m->ctx, p, [&](auto R, auto S, dim3 g, dim3 b) {
+            periodic_stage_kernel<decltype(R)::value, decltype(S)::value><<<g, b, 0, m->ctx->stream>>>(
               p->dev, c[0], c[1], c[2], c[3], c[4], NVD(ym1), NVD(ym2), NVD(y), NVD(F), NVD(yj));
           });
         }
@@ -1711,7 +1719,7 @@ static int evolve_generic(LSRKMem* m, double tout, double clip, int itask)
         STS_Context ctx = m->ctx;
         STS_Problem p = (STS_Problem)m->user_data;
         slot_arm(ctx, SLOT_GENERIC);
-        periodic_rows(ctx, p, [&](auto R, dim3 g, dim3 b) {
+        periodic_rows(ctx, p, [&](auto R, auto, dim3 g, dim3 b) {
           periodic_end_kernel<decltype(R)::value><<<g, b, 0, ctx->stream>>>(
             p->dev, NVD(y), NVD(yj), NVD(F), NVD(m->g_Fnew), 0.4 * h, m->rtol, m->atol, ctx->d_work,
             ctx->d_slots + SLOT_GENERIC);

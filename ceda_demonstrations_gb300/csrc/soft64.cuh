@@ -235,4 +235,25 @@ __device__ __forceinline__ float s64_to_float(double x)
   if (soft64::to_float(x, &f)) return f;
   return __double2float_rn(x);
 }
+// SOFT false: the FP64 instruction (kernels that latency bounds, see their rules)
+template <bool SOFT>
+__device__ __forceinline__ double s64_add(double a, double b)
+{
+  return SOFT ? s64_add(a, b) : __dadd_rn(a, b);
+}
+template <bool SOFT>
+__device__ __forceinline__ double s64_mul(const soft64::Factor& f, double a, double b)
+{
+  return SOFT ? s64_mul(f, a, b) : __dmul_rn(a, b);
+}
+template <bool SOFT>
+__device__ __forceinline__ double s64_mul(double a, double b)
+{
+  return SOFT ? s64_mul(a, b) : __dmul_rn(a, b);
+}
+template <bool SOFT>
+__device__ __forceinline__ double s64_fma_small(const soft64::Factor& f, double a, double b, double c)
+{
+  return SOFT ? s64_fma_small(f, a, b, c) : __fma_rn(a, b, c);
+}
 #endif

@@ -563,3 +563,21 @@ def test_mixed_default_groups_on_odd_rows_bitwise(ctx, stslib, oracle, tmp_path,
     I.evolve(t2, y)
     K.evolve(t2, z)
     assert np.array_equal(y.numpy(), z.numpy()) and I.stats()["nst"] == K.stats()["nst"]
+
+
+@pytest.mark.parametrize("kind", [1, 2])
+@pytest.mark.parametrize("nx,ny", [(311, 250), (312, 250), (389, 400), (390, 400)])
+def test_stage_arithmetic_rule_bitwise(ctx, stslib, oracle, kind, nx, ny):
+    """FP64 stages on both sides of the two size rules (77 824 points: FP64 or integer products,
+    155 648: rows per thread; 152 SMs), Dirichlet and periodic, against the oracle bit for bit."""
+    pk = dict(kind=kind, nx=nx, ny=ny, kx=1.0, ky=0.3, inhomogeneous=kind == 2)
+    P, O = stslib.Problem(ctx, **pk), oracle.Problem(**pk)
+    y0 = np.random.default_rng(nx).standard_normal(nx * ny)
+    h = 30.0 / (8.0 * max(nx * nx, ny * ny))
+    I = stslib.LSRKStep(ctx, P, 0.0, stslib.NVector.from_numpy(ctx, y0), method=1, rtol=1e-6, atol=1e-10, hfixed=h)
+    J = oracle.Integrator(O, y0.copy(), method=1, rtol=1e-6, atol=1e-10, hfixed=h)
+    y = P.vector()
+    I.evolve(h, y)
+    assert J.evolve(h) == 0
+    assert I.stats()["nst"] == 1
+    assert np.array_equal(y.numpy(), J.y)
