@@ -171,9 +171,7 @@ static int ark_atimes(void* d, N_Vector v, N_Vector out)
   ARKStepMem* m = AM(d);
   m->njv++;
   if (m->f == STS_Diffusion)
-  {
-    if (STS_JacTimes(v, m->tmp, m->cur_t, nullptr, nullptr, m->user_data, nullptr)) return -1;
-  }
+    return sts_shift((STS_Problem)m->user_data, m->cur_gamma, v, out);
   else
   { // difference quotient at the current iterate: (f(t, z + sig v) - f(t, z)) / sig,
     // sig = 1 / ||v||_WRMS

@@ -44,6 +44,7 @@ struct StepArgs {
 // ---------------------------------------------------------------------------------------
 // point operators
 // ---------------------------------------------------------------------------------------
+template <bool SOFT = false> // the center product as integer code (soft64.cuh)
 __device__ __forceinline__ double dirichlet_point(const ProbDev& P, const double* __restrict__ u,
                                                   long long i, long long j)
 {
@@ -54,7 +55,7 @@ __device__ __forceinline__ double dirichlet_point(const ProbDev& P, const double
   const double us   = (j > 0) ? u[k - P.nx] : 0.0;
   const double un   = (j < P.ny - 1) ? u[k + P.nx] : 0.0;
   const double sx = uw + ue, sy = us + un;
-  double acc = P.cc * uc;
+  double acc = s64_mul<SOFT>(P.cc, uc);
   acc        = __fma_rn(P.cx, sx, acc);
   acc        = __fma_rn(P.cy, sy, acc);
   return acc;

@@ -798,14 +798,11 @@ namespace {
 struct ShiftedOp {
   STS_Problem p;
   double gamma;
-  N_Vector tmp;
 };
 int shifted_atimes(void* d, N_Vector v, N_Vector z)
 {
   ShiftedOp* a = (ShiftedOp*)d;
-  if (STS_JacTimes(v, a->tmp, 0.0, nullptr, nullptr, a->p, nullptr)) return -1;
-  N_VLinearSum_Sts(1.0, v, -a->gamma, a->tmp, z);
-  return 0;
+  return sts_shift(a->p, a->gamma, v, z);
 }
 int jacobi_psolve(void* d, N_Vector r, N_Vector z, double tol, int lr)
 {
@@ -820,7 +817,7 @@ extern "C" int STS_SDIRK2EvolveLS(STS_Problem p, void* LS, int precond, N_Vector
   STS_MARK_FUNCTION;
   LinSol* L = (LinSol*)LS;
   if (!p || !L || !y) return -1;
-  ShiftedOp op{p, 0.0, N_VClone_Sts(y)};
+  ShiftedOp op{p, 0.0};
   STS_SUNLinSolSetATimes(L, &op, shifted_atimes);
   STS_SUNLinSolSetPreconditioner(L, precond ? &op : nullptr, precond ? jacobi_psolve : nullptr);
   const int rc = sdirk2_run(p, y, t0, h, nsteps, total_iters, [&](double hg, N_Vector rhs, N_Vector d, int* it) {
@@ -831,7 +828,6 @@ extern "C" int STS_SDIRK2EvolveLS(STS_Problem p, void* LS, int precond, N_Vector
   });
   STS_SUNLinSolSetATimes(L, nullptr, nullptr);
   STS_SUNLinSolSetPreconditioner(L, nullptr, nullptr);
-  N_VDestroy_Sts(op.tmp);
   return rc;
 }
 
@@ -852,7 +848,7 @@ extern "C" int STS_ImplicitSolveLS(STS_Problem p, double gamma, void* LS, int pr
                   "preconditioning type)");
     return -1;
   }
-  ShiftedOp op{p, gamma, N_VClone_Sts(b)};
+  ShiftedOp op{p, gamma};
   STS_SUNLinSolSetATimes(L, &op, shifted_atimes);
   if (prec == 1) STS_SUNLinSolSetPreconditioner(L, &op, jacobi_psolve);
   else if (prec == 2) STS_SUNLinSolSetPreconditioner(L, P_data, psolve);
@@ -862,7 +858,6 @@ extern "C" int STS_ImplicitSolveLS(STS_Problem p, double gamma, void* LS, int pr
   if (relres) *relres = STS_SUNLinSolResNorm(L);
   STS_SUNLinSolSetATimes(L, nullptr, nullptr);
   STS_SUNLinSolSetPreconditioner(L, nullptr, nullptr);
-  N_VDestroy_Sts(op.tmp);
   return rc;
 }
 

@@ -832,23 +832,10 @@ struct ShiftOp {
   STS_Problem p;
   double gamma;
 };
-// z = v - gamma A v, the operations of STS_JacTimes and N_VLinearSum(1, v, -gamma, A v) in one pass
-__global__ void shift_kernel(ProbDev P, double gamma, const double* __restrict__ v, double* __restrict__ z)
-{
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long j = (long long)blockIdx.y * blockDim.y + threadIdx.y;
-  if (i >= P.nx || j >= P.ny) return;
-  const double t = P.kind == STS_PROBLEM_PERIODIC ? periodic_point(P, v, i, j) : dirichlet_point(P, v, i, j);
-  z[j * P.nx + i] = __dadd_rn(v[j * P.nx + i], s64_mul(-gamma, t));
-}
 int shift_atimes(void* d, N_Vector v, N_Vector z)
 {
   ShiftOp* a = (ShiftOp*)d;
-  if (NVL(v) != a->p->nx * a->p->ny || NVL(z) != NVL(v)) return -1;
-  const dim3 b(32, 8);
-  ctx_activate(a->p->ctx);
-  shift_kernel<<<blocks2d(a->p->nx, a->p->ny, b), b, 0, a->p->ctx->stream>>>(a->p->dev, a->gamma, NVD(v), NVD(z));
-  return STS_CUDA_OK(cudaGetLastError()) ? 0 : -1;
+  return sts_shift(a->p, a->gamma, v, z);
 }
 } // namespace
 

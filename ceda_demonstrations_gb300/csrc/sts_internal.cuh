@@ -294,6 +294,8 @@ inline long long NVL(N_Vector v) { return NVC(v)->length; }
 
 // problem-level kernels used by the integrator and the solvers (diffusion.cu)
 int sts_rhs_launch(STS_Problem p, double t, const double* u, double* f, bool forcing, cudaStream_t s);
+// z = v - gamma A v of the built-in problem (v and z distinct)
+int sts_shift(STS_Problem p, double gamma, N_Vector v, N_Vector z);
 double sts_dot_exact(STS_Context ctx, const double* x, const double* y, long long n, int slot);
 double sts_wrms_ewt(STS_Context ctx, const double* a, const double* b, const double* y, long long n,
                     double rtol, double atol, int slot);
