@@ -41,6 +41,7 @@ __device__ __forceinline__ void krylov_block_finish(xsum::Limbs* a, unsigned* fl
   if (tid == xsum::NL + 1) s->ticket = 0u;
 #pragma unroll
   for (int c = 0; c < NACC; ++c) f[c] = __shfl_sync(0xffffffffu, f[c], xsum::NL);
+  __syncwarp(); // lane 0 reads the other lanes' limbs: a shuffle orders no memory
   if (tid == 0)
   {
     double r[NACC];

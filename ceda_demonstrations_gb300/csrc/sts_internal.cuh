@@ -215,6 +215,7 @@ __device__ __forceinline__ void xsum_block_finish(xsum::Limbs& a, unsigned flags
   else if (tid == xsum::NL) fl = atomicExch(&w->flags, 0u);
   else if (tid == xsum::NL + 1) w->ticket = 0u;
   fl = __shfl_sync(0xffffffffu, fl, xsum::NL);
+  __syncwarp(); // lane 0 reads the other lanes' limbs: a shuffle orders no memory
   if (tid == 0)
   {
     double r = xsum::finalize(sm[0], fl);
