@@ -461,12 +461,15 @@ extern "C" int N_VDotProdMulti_Sts(int nvec, N_Vector x, N_Vector* Y, double* do
   long long n     = NVL(x);
   ctx_activate(ctx);
   constexpr int CH = STS_NSLOTS - SLOT_MULTI;
+  // every length before the first launch: a return with reductions in flight would let a later call
+  // arm their slots and take their results for its own
+  for (int k = 0; k < nvec; ++k)
+    if (NVL(Y[k]) != n) return -1;
   for (int c0 = 0; c0 < nvec; c0 += CH)
   {
     const int cnt = std::min(CH, nvec - c0);
     for (int k = 0; k < cnt; ++k)
     {
-      if (NVL(Y[c0 + k]) != n) return -1;
       slot_arm(ctx, SLOT_MULTI + k);
       xred_kernel<0><<<red_blocks(ctx, n), 256, 0, ctx->stream>>>(n, NVD(x), NVD(Y[c0 + k]), ctx->d_work,
                                                                            ctx->d_slots + SLOT_MULTI + k);
