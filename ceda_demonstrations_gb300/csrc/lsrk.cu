@@ -270,6 +270,7 @@ struct LSRKMem {
   float* Ffb[2] = {nullptr, nullptr}; // FP32 copies (mixed)
   double* Y[3]  = {nullptr, nullptr, nullptr};
   float* D[4]   = {nullptr, nullptr, nullptr, nullptr}; // D[3]: fused stages only
+  size_t Ffb_bytes[2] = {}, D_bytes[4] = {};            // allocated sizes
   double* evec  = nullptr;
   float* per_faces = nullptr; // mixed reference mode: FP32 Dxw | Dxe | Dys | Dyn
   int par       = 0; // current parity: yb[par] = y_n
@@ -516,6 +517,19 @@ static size_t f32_field_bytes(const LSRKMem* m)
   return (size_t)(p->dev.ldf * p->ny) * sizeof(float);
 }
 
+// an FP32 buffer of at least `bytes` (the periodic path needs n floats, the fused one ldf * ny of
+// its grid); a new one is zeroed
+static bool fit_f32(LSRKMem* m, float** b, size_t* have, size_t bytes)
+{
+  if (*b && *have >= bytes) return true;
+  cudaFree(*b);
+  *b    = nullptr;
+  *have = 0;
+  if (!STS_CUDA_OK(cudaMalloc(b, bytes))) return false;
+  *have = bytes;
+  return STS_CUDA_OK(cudaMemsetAsync(*b, 0, bytes, m->ctx->stream));
+}
+
 // allocate the fused-path buffers (y0 copied into yb[0])
 static int alloc_fused(LSRKMem* m, const double* y0dev)
 {
@@ -524,7 +538,7 @@ static int alloc_fused(LSRKMem* m, const double* y0dev)
   for (int b = 0; b < 2; ++b)
   {
     if (!STS_CUDA_OK(cudaMalloc(&m->yb[b], n8)) || !STS_CUDA_OK(cudaMalloc(&m->Fb[b], n8)) ||
-        !STS_CUDA_OK(cudaMalloc(&m->Ffb[b], n4)) || !STS_CUDA_OK(cudaMemsetAsync(m->Ffb[b], 0, n4, st)))
+        !fit_f32(m, &m->Ffb[b], &m->Ffb_bytes[b], n4))
       return -1;
   }
   m->par_bytes = sizeof(StepArgs) + 8 + sizeof(StageArgs) * (size_t)(m->smax + 1);
@@ -539,28 +553,23 @@ static int alloc_fused(LSRKMem* m, const double* y0dev)
   return 0;
 }
 
-// after ARKodeSetUserData with a problem of another grid shape (the same number of points): FP32
-// buffers of that shape's pitch, with the FP32 copy of F_n
+// After ARKodeSetUserData with a problem of another grid shape (the same number of points), or where
+// the mixed periodic path has left its smaller buffers: FP32 buffers of the grid's pitch, with the FP32
+// copy of F_n. Whatever touches Ffb or D calls this first.
 static int refit_f32(LSRKMem* m)
 {
-  STS_Problem p = (STS_Problem)m->user_data;
-  if (m->f32_nx == p->nx && m->f32_ny == p->ny) return 0;
+  STS_Problem p   = (STS_Problem)m->user_data;
+  const size_t n4 = f32_field_bytes(m);
+  bool fits       = m->f32_nx == p->nx && m->f32_ny == p->ny;
+  for (int b = 0; b < 4; ++b) fits = fits && (!m->D[b] || m->D_bytes[b] >= n4);
+  if (fits) return 0;
   if (!STS_CUDA_OK(cudaStreamSynchronize(m->ctx->stream))) return -1;
   for (auto& kv : m->graphs) cudaGraphExecDestroy(kv.second);
   m->graphs.clear();
   for (int b = 0; b < 4; ++b)
-  {
-    cudaFree(m->D[b]);
-    m->D[b] = nullptr;
-  }
-  const size_t n4 = f32_field_bytes(m);
+    if (m->D[b] && !fit_f32(m, &m->D[b], &m->D_bytes[b], n4)) return -1;
   for (int b = 0; b < 2; ++b)
-  {
-    cudaFree(m->Ffb[b]);
-    m->Ffb[b] = nullptr;
-    if (!STS_CUDA_OK(cudaMalloc(&m->Ffb[b], n4)) || !STS_CUDA_OK(cudaMemsetAsync(m->Ffb[b], 0, n4, m->ctx->stream)))
-      return -1;
-  }
+    if (!fit_f32(m, &m->Ffb[b], &m->Ffb_bytes[b], n4)) return -1;
   if (m->mixed && m->initialized) field_to_f32(m->ctx, p, m->Fb[m->par], m->Ffb[m->par]);
   m->tma.ok = m->tma.fz_ok = false;
   m->tuned  = false;
@@ -576,7 +585,7 @@ static int ensure_stage_buffers(LSRKMem* m)
   for (int b = 0; b < 3; ++b)
   {
     if (!m->mixed && !m->Y[b] && !STS_CUDA_OK(cudaMalloc(&m->Y[b], n8))) return -1;
-    if (m->mixed && !m->D[b] && !STS_CUDA_OK(cudaMalloc(&m->D[b], n4))) return -1;
+    if (m->mixed && !fit_f32(m, &m->D[b], &m->D_bytes[b], n4)) return -1;
   }
   // fused stages need a fourth buffer (a group reads two and writes two); the tensor maps of
   // the single-stage and the fused kernels cover every allocated buffer
@@ -586,7 +595,7 @@ static int ensure_stage_buffers(LSRKMem* m)
     STS_Problem p = (STS_Problem)m->user_data;
     if (tma_stage32_supported(p->nx, p->ny))
     {
-      if (want_fused && !m->D[3] && !STS_CUDA_OK(cudaMalloc(&m->D[3], n4))) return -1;
+      if (want_fused && !fit_f32(m, &m->D[3], &m->D_bytes[3], n4)) return -1;
       if (tma_stage32_prepare(&m->tma, m->D, m->Ffb, p->nx, p->ny) && want_fused)
         tma_fused_prepare(&m->tma, m->D, m->Ffb, p->nx, p->ny);
     }
@@ -1649,8 +1658,8 @@ static int evolve_generic(LSRKMem* m, double tout, double clip, int itask)
         {
           if (!STS_CUDA_OK(cudaMalloc(&m->per_faces, (2 * p->nx + 2 * p->ny) * sizeof(float)))) return STS_ERR_FAILURE;
           for (int b = 0; b < 3; ++b)
-            if (!m->D[b] && !STS_CUDA_OK(cudaMalloc(&m->D[b], n * sizeof(float)))) return STS_ERR_FAILURE;
-          if (!m->Ffb[0] && !STS_CUDA_OK(cudaMalloc(&m->Ffb[0], n * sizeof(float)))) return STS_ERR_FAILURE;
+            if (!fit_f32(m, &m->D[b], &m->D_bytes[b], n * sizeof(float))) return STS_ERR_FAILURE;
+          if (!fit_f32(m, &m->Ffb[0], &m->Ffb_bytes[0], n * sizeof(float))) return STS_ERR_FAILURE;
           sts_f64_to_f32(ctx, p->dev.Dxw, m->per_faces, p->nx);
           sts_f64_to_f32(ctx, p->dev.Dxe, m->per_faces + p->nx, p->nx);
           sts_f64_to_f32(ctx, p->dev.Dys, m->per_faces + 2 * p->nx, p->ny);
@@ -2166,6 +2175,7 @@ extern "C" int STS_ARKodeReset(void* mem, double t, N_Vector y)
   m->interp_ready = false;
   if (fused(m) && m->yb[0])
   {
+    if (refit_f32(m)) return STS_ERR_FAILURE;
     if (!STS_CUDA_OK(cudaMemcpyAsync(m->yb[m->par], NVD(y), m->n * sizeof(double), cudaMemcpyDeviceToDevice,
                                      m->ctx->stream)))
       return STS_ERR_FAILURE;
@@ -2196,6 +2206,9 @@ extern "C" int STS_LSRKStepTimeStageKernel(void* mem, int nlaunch, double* ms_pe
   ctx_activate(m->ctx);
   STS_Problem p   = (STS_Problem)m->user_data;
   cudaStream_t st = m->ctx->stream;
+  // (the problem may have changed since the last step, or the step lie in a checkpoint)
+  if (!m->yb[0] || ensure_stage_buffers(m) || ensure_par(m)) return STS_ERR_FAILURE;
+  if (m->mixed && !m->tuned) autotune_stage32(m, p);
   const int j     = m->last_s / 2 > 2 ? m->last_s / 2 : 2;
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
@@ -2419,14 +2432,14 @@ extern "C" int STS_LSRKStepWriteCheckpoint(void* mem, const char* path)
   if (!path) return STS_ILL_INPUT;
   ctx_activate(m->ctx);
   cudaStream_t st = m->ctx->stream;
-  if (!STS_CUDA_OK(cudaStreamSynchronize(st))) return STS_ERR_FAILURE;
+  const bool fz   = fused(m) && m->yb[0] != nullptr;
+  if ((fz && refit_f32(m)) || !STS_CUDA_OK(cudaStreamSynchronize(st))) return STS_ERR_FAILURE;
   CkptHeader h;
   memset(&h, 0, sizeof(h));
   memcpy(h.magic, CKPT_MAGIC, 8);
   h.version         = 1;
   h.method          = m->method;
   h.mixed           = m->mixed;
-  const bool fz     = fused(m) && m->yb[0] != nullptr;
   h.fused_path      = fz;
   h.n               = m->n;
   h.t               = m->t;
@@ -2501,7 +2514,7 @@ extern "C" int STS_LSRKStepReadCheckpoint(void* mem, const char* path)
     sts_set_error("STS_LSRKStepReadCheckpoint: checkpoint written by the %s path", h.fused_path ? "fused" : "generic");
     return STS_ILL_INPUT;
   }
-  if (fz && !m->yb[0] && alloc_fused(m, NVD(m->g_y)))
+  if (fz && (m->yb[0] ? refit_f32(m) : alloc_fused(m, NVD(m->g_y))))
   {
     fclose(f);
     return STS_ERR_FAILURE;

@@ -1,0 +1,96 @@
+"""ARKodeSetUserData hands an integrator that has stepped another problem with as many points: every call
+that may come next works on the new problem alone, bit for bit as an integrator created for it."""
+import numpy as np
+import pytest
+
+import ceda_demonstrations_gb300 as sts
+
+pytestmark = pytest.mark.gpu
+H = 2e-4
+
+
+def make(ctx, kind, nx, ny, ky=0.3):
+    """A problem whose spectral radius stays below the bound that the integrators are given."""
+    kx = min(1.0, 1e5 / max(nx, ny) ** 2)
+    return sts.Problem(ctx, kind, nx, ny, kx, ky * kx, inhomogeneous=kind == sts.PERIODIC)
+
+
+def state(ctx, P, seed=1):
+    return sts.NVector.from_numpy(ctx, np.random.default_rng(seed).standard_normal(P.nx * P.ny))
+
+
+def integrator(ctx, P, y0, mixed):
+    """Fixed steps of the same stage count on either problem, whatever ran before."""
+    return sts.LSRKStep(ctx, P, 0.0, y0, method=sts.RKL, mixed=mixed, hfixed=H, dom_eig=lambda t: -6e5)
+
+
+def run(I, P, t):
+    y = P.vector()
+    I.set_stop_time(t)
+    I.evolve(t, y)
+    return y.numpy()
+
+
+def switch(I, P):
+    assert sts.lib().STS_ARKodeSetUserData(I.mem, P.h) == 0
+
+
+# rows of the first shape need no padding in the FP32 fields, of the second two or three columns
+SHAPES = [((40, 21), (42, 20)), ((120, 70), (105, 80)), ((1200, 700), (1050, 800))]
+
+
+@pytest.mark.parametrize("mixed", [False, True])
+@pytest.mark.parametrize("shapes", SHAPES, ids=str)
+def test_another_shape_then_reset(ctx, shapes, mixed):
+    A, B = (make(ctx, sts.MANUFACTURED, *s) for s in shapes)
+    I = integrator(ctx, A, state(ctx, A), mixed)
+    ya = run(I, A, 2 * H)
+    y1 = state(ctx, B, 2)
+    switch(I, B)
+    I.reset(0.0, y1)
+    assert np.array_equal(run(I, B, 3 * H), run(integrator(ctx, B, y1, mixed), B, 3 * H))
+    switch(I, A)  # and back
+    I.reset(0.0, state(ctx, A))
+    assert np.array_equal(run(I, A, 2 * H), ya)
+
+
+@pytest.mark.parametrize("mixed", [False, True])
+@pytest.mark.parametrize("shapes", SHAPES, ids=str)
+def test_another_shape_then_checkpoint(ctx, tmp_path, shapes, mixed):
+    A, B = (make(ctx, sts.MANUFACTURED, *s) for s in shapes)
+    # reading one
+    J = integrator(ctx, B, state(ctx, B, 2), mixed)
+    run(J, B, 2 * H)
+    J.write_checkpoint(str(tmp_path / "b"))
+    yb = run(J, B, 4 * H)
+    I = integrator(ctx, A, state(ctx, A), mixed)
+    run(I, A, 2 * H)
+    switch(I, B)
+    I.read_checkpoint(str(tmp_path / "b"))
+    assert np.array_equal(run(I, B, 4 * H), yb)
+    # writing one: it holds what the integrator continues from
+    K = integrator(ctx, A, state(ctx, A), mixed)
+    run(K, A, 2 * H)
+    switch(K, B)
+    K.write_checkpoint(str(tmp_path / "k"))
+    L = integrator(ctx, B, state(ctx, B, 2), mixed)
+    L.read_checkpoint(str(tmp_path / "k"))
+    assert np.array_equal(run(K, B, 4 * H), run(L, B, 4 * H))
+
+
+@pytest.mark.parametrize("mixed", [False, True])
+def test_stage_timing_after_a_change_and_a_checkpoint(ctx, tmp_path, mixed):
+    A, B = make(ctx, sts.MANUFACTURED, 120, 70), make(ctx, sts.MANUFACTURED, 105, 80)
+    I = integrator(ctx, A, state(ctx, A), mixed)
+    run(I, A, 2 * H)
+    I.write_checkpoint(str(tmp_path / "a"))
+    want = run(I, A, 4 * H)
+    J = integrator(ctx, A, state(ctx, A), mixed)
+    J.read_checkpoint(str(tmp_path / "a"))
+    assert J.time_stage_kernel(3) > 0.0  # no stage has run in this integrator
+    assert np.array_equal(run(J, A, 4 * H), want)
+    switch(I, B)
+    assert I.time_stage_kernel(3) > 0.0
+    y1 = state(ctx, B, 2)
+    I.reset(0.0, y1)
+    assert np.array_equal(run(I, B, 3 * H), run(integrator(ctx, B, y1, mixed), B, 3 * H))
