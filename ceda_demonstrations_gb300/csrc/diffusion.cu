@@ -9,6 +9,7 @@
 // operations (the library is compiled with --fmad=false), in the order the CPU oracle uses.
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cmath>
 #include <cstdlib>
 #include <vector>
@@ -50,8 +51,10 @@ extern "C" STS_Problem STS_ProblemCreate(STS_Context ctx, int kind, sts_index nx
     return nullptr;
   }
   ctx_activate(ctx);
+  static std::atomic<unsigned long long> created{0};
   STS_Problem p = new STS_Problem_();
   p->ctx        = ctx;
+  p->serial     = ++created;
   p->kind       = kind;
   p->inhom      = (kind == STS_PROBLEM_PERIODIC) ? inhomogeneous : 0;
   p->nx         = nx;

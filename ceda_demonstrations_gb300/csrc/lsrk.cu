@@ -249,6 +249,7 @@ struct LSRKMem {
   // the rest of a step runs in groups of fuse_ks
   int deep_ti    = -1;
   double deep_ms = 0.0;
+  unsigned long long kept_for = 0;  // STS_Problem_::serial that `graphs` and `per_faces` hold for
   long long f32_nx = 0, f32_ny = 0; // the grid that the FP32 buffers and their tensor maps fit
   long long n           = 0;
 
@@ -515,6 +516,21 @@ static size_t f32_field_bytes(const LSRKMem* m)
 {
   const STS_Problem p = (STS_Problem)m->user_data;
   return (size_t)(p->dev.ldf * p->ny) * sizeof(float);
+}
+
+// Recorded steps hold the problem's coefficients, tables and kind, per_faces its face coefficients:
+// both go when ARKodeSetUserData has handed over another problem.
+static bool adopt_problem(LSRKMem* m)
+{
+  const STS_Problem p = (STS_Problem)m->user_data;
+  if (m->rhs != STS_Diffusion || !p || m->kept_for == p->serial) return true;
+  if (!STS_CUDA_OK(cudaStreamSynchronize(m->ctx->stream))) return false;
+  for (auto& kv : m->graphs) cudaGraphExecDestroy(kv.second);
+  m->graphs.clear();
+  cudaFree(m->per_faces);
+  m->per_faces = nullptr;
+  m->kept_for  = p->serial;
+  return true;
 }
 
 // an FP32 buffer of at least `bytes` (the periodic path needs n floats, the fused one ldf * ny of
@@ -2135,6 +2151,7 @@ extern "C" int STS_ARKodeEvolve(void* mem, double tout, N_Vector yout, double* t
   // start every evolve from a clean reduction workspace (a failed launch could leave it dirty)
   cudaMemsetAsync(m->ctx->d_work, 0, sizeof(RedWork), st);
   const double clip = m->tstopset ? m->tstop : INFINITY;
+  if (!adopt_problem(m)) return STS_ERR_FAILURE;
   int ret;
   if (fused(m))
   {

@@ -264,6 +264,7 @@ __device__ __forceinline__ bool sts_in_bounds(bool ok, int* err)
 
 struct STS_Problem_ {
   STS_Context ctx = nullptr;
+  unsigned long long serial = 0; // another number for every problem created (addresses come again)
   int kind = 0, inhom = 0;
   long long nx = 0, ny = 0;
   double kx = 1, ky = 1, xl = 0, xu = 1, yl = 0, yu = 1, dx = 0, dy = 0, cx = 0, cy = 0, cc = 0;

@@ -94,3 +94,34 @@ def test_stage_timing_after_a_change_and_a_checkpoint(ctx, tmp_path, mixed):
     y1 = state(ctx, B, 2)
     I.reset(0.0, y1)
     assert np.array_equal(run(I, B, 3 * H), run(integrator(ctx, B, y1, mixed), B, 3 * H))
+
+
+SAME = [(sts.MANUFACTURED, 0.3, sts.MANUFACTURED, 0.05), (sts.MANUFACTURED, 0.3, sts.UNFORCED, 0.3),
+        (sts.UNFORCED, 0.1, sts.MANUFACTURED, 0.2), (sts.PERIODIC, 0.3, sts.PERIODIC, 0.05)]
+
+
+@pytest.mark.parametrize("mixed", [False, True])
+@pytest.mark.parametrize("case", SAME, ids=str)
+def test_same_shape_other_coefficients_or_kind(ctx, case, mixed):
+    """Steps recorded for one problem, and the FP32 faces of a periodic one, are not used for another."""
+    A, B = make(ctx, case[0], 120, 70, case[1]), make(ctx, case[2], 120, 70, case[3])
+    I = integrator(ctx, A, state(ctx, A), mixed)
+    ya = run(I, A, 3 * H)
+    y1 = state(ctx, B, 2)
+    switch(I, B)
+    I.reset(0.0, y1)
+    assert np.array_equal(run(I, B, 3 * H), run(integrator(ctx, B, y1, mixed), B, 3 * H))
+    switch(I, A)
+    I.reset(0.0, state(ctx, A))
+    assert np.array_equal(run(I, A, 3 * H), ya)
+
+
+@pytest.mark.parametrize("mixed", [False, True])
+def test_periodic_problem_of_another_shape(ctx, mixed):
+    A, B = make(ctx, sts.PERIODIC, 105, 80), make(ctx, sts.PERIODIC, 84, 100)
+    I = integrator(ctx, A, state(ctx, A), mixed)
+    run(I, A, 2 * H)
+    y1 = state(ctx, B, 2)
+    switch(I, B)
+    I.reset(0.0, y1)
+    assert np.array_equal(run(I, B, 3 * H), run(integrator(ctx, B, y1, mixed), B, 3 * H))
