@@ -275,6 +275,7 @@ struct LSRKMem {
   double* evec  = nullptr;
   float* per_faces = nullptr; // mixed reference mode: FP32 Dxw | Dxe | Dys | Dyn
   int par       = 0; // current parity: yb[par] = y_n
+  bool state_fused = false; // the state is in yb / Fb, not in g_y / g_Fn
   N_Vector nv_y = nullptr, nv_F = nullptr, nv_tmp[3] = {nullptr, nullptr, nullptr};
 
   // stage parameters: [StepArgs][StageArgs x (smax+1)] on the device and pinned on the host
@@ -518,21 +519,6 @@ static size_t f32_field_bytes(const LSRKMem* m)
   return (size_t)(p->dev.ldf * p->ny) * sizeof(float);
 }
 
-// Recorded steps hold the problem's coefficients, tables and kind, per_faces its face coefficients:
-// both go when ARKodeSetUserData has handed over another problem.
-static bool adopt_problem(LSRKMem* m)
-{
-  const STS_Problem p = (STS_Problem)m->user_data;
-  if (m->rhs != STS_Diffusion || !p || m->kept_for == p->serial) return true;
-  if (!STS_CUDA_OK(cudaStreamSynchronize(m->ctx->stream))) return false;
-  for (auto& kv : m->graphs) cudaGraphExecDestroy(kv.second);
-  m->graphs.clear();
-  cudaFree(m->per_faces);
-  m->per_faces = nullptr;
-  m->kept_for  = p->serial;
-  return true;
-}
-
 // an FP32 buffer of at least `bytes` (the periodic path needs n floats, the fused one ldf * ny of
 // its grid); a new one is zeroed
 static bool fit_f32(LSRKMem* m, float** b, size_t* have, size_t bytes)
@@ -571,7 +557,7 @@ static int alloc_fused(LSRKMem* m, const double* y0dev)
 
 // After ARKodeSetUserData with a problem of another grid shape (the same number of points), or where
 // the mixed periodic path has left its smaller buffers: FP32 buffers of the grid's pitch, with the FP32
-// copy of F_n. Whatever touches Ffb or D calls this first.
+// copy of F_n.
 static int refit_f32(LSRKMem* m)
 {
   STS_Problem p   = (STS_Problem)m->user_data;
@@ -594,9 +580,72 @@ static int refit_f32(LSRKMem* m)
   return 0;
 }
 
+// the generic path's temporaries
+static void alloc_generic(LSRKMem* m)
+{
+  if (m->g_Y[0]) return;
+  N_Vector y = m->g_y;
+  for (int k = 0; k < 3; ++k) m->g_Y[k] = N_VClone_Sts(y);
+  m->g_F    = N_VClone_Sts(y);
+  m->g_Fnew = N_VClone_Sts(y);
+  m->g_err  = N_VClone_Sts(y);
+  m->g_ewt  = N_VClone_Sts(y);
+  m->g_yold = N_VClone_Sts(y);
+  m->g_Fold = N_VClone_Sts(y);
+}
+
+// Called first by whatever uses the state or the buffers: ARKodeSetUserData may have handed over another
+// problem since.
+// - Recorded steps hold the problem's coefficients, tables and kind, per_faces its face coefficients:
+//   both go with it.
+// - The state is in yb / Fb (fused path) or in g_y / g_Fn (generic path): it moves where the problem's
+//   path keeps it, with y_old of the last step (these methods' dense output needs no F).
+// - The FP32 buffers get the grid's pitch.
+static bool adopt_problem(LSRKMem* m)
+{
+  const STS_Problem p = (STS_Problem)m->user_data;
+  if (m->rhs != STS_Diffusion || !p) return true;
+  cudaStream_t st = m->ctx->stream;
+  if (m->kept_for != p->serial)
+  {
+    if (!STS_CUDA_OK(cudaStreamSynchronize(st))) return false;
+    for (auto& kv : m->graphs) cudaGraphExecDestroy(kv.second);
+    m->graphs.clear();
+    cudaFree(m->per_faces);
+    m->per_faces = nullptr;
+    m->kept_for  = p->serial;
+  }
+  const bool fz = fused(m);
+  if (fz != m->state_fused)
+  {
+    const size_t n8 = m->n * sizeof(double);
+    auto move       = [&](double* parity, N_Vector v) {
+      double* g = NVD(v);
+      return STS_CUDA_OK(cudaMemcpyAsync(fz ? parity : g, fz ? g : parity, n8, cudaMemcpyDeviceToDevice, st));
+    };
+    if (fz && !m->yb[0])
+    {
+      if (alloc_fused(m, NVD(m->g_y))) return false;
+    }
+    else if (!move(m->yb[m->par], m->g_y)) return false;
+    if (m->initialized && !move(m->Fb[m->par], m->g_Fn)) return false;
+    if (m->interp_ready)
+    {
+      alloc_generic(m);
+      if (!move(m->yb[1 - m->par], m->g_yold)) return false;
+    }
+    m->state_fused = fz;
+    if (fz && m->mixed && m->initialized)
+    {
+      if (refit_f32(m)) return false;
+      field_to_f32(m->ctx, p, m->Fb[m->par], m->Ffb[m->par]);
+    }
+  }
+  return !fz || refit_f32(m) == 0;
+}
+
 static int ensure_stage_buffers(LSRKMem* m)
 {
-  if (refit_f32(m)) return -1;
   const size_t n8 = m->n * sizeof(double), n4 = f32_field_bytes(m);
   for (int b = 0; b < 3; ++b)
   {
@@ -1563,16 +1612,7 @@ static bool periodic_fusable(const LSRKMem* m)
 static int evolve_generic(LSRKMem* m, double tout, double clip, int itask)
 {
   N_Vector y = m->g_y, F = m->g_Fn;
-  if (!m->g_Y[0])
-  {
-    for (int k = 0; k < 3; ++k) m->g_Y[k] = N_VClone_Sts(y);
-    m->g_F    = N_VClone_Sts(y);
-    m->g_Fnew = N_VClone_Sts(y);
-    m->g_err  = N_VClone_Sts(y);
-    m->g_ewt  = N_VClone_Sts(y);
-    m->g_yold = N_VClone_Sts(y);
-    m->g_Fold = N_VClone_Sts(y);
-  }
+  alloc_generic(m);
   if (!m->initialized)
   {
     if (m->rhs(m->t, y, F, m->user_data) != 0) return STS_RHSFUNC_FAIL;
@@ -2086,7 +2126,7 @@ static int lsrk_interp_degree(const LSRKMem* m)
 
 static int lsrk_output(LSRKMem* m, N_Vector yout, double tq, bool interp)
 {
-  const bool fz      = fused(m) && m->yb[0];
+  const bool fz      = m->state_fused;
   const double* ycur = fz ? m->yb[m->par] : NVD(m->g_y);
   cudaStream_t st    = m->ctx->stream;
   if (!interp || tq == m->t)
@@ -2131,6 +2171,7 @@ extern "C" int STS_ARKodeEvolve(void* mem, double tout, N_Vector yout, double* t
     m->tretlast = tr;
     return ret;
   };
+  if (!adopt_problem(m)) return STS_ERR_FAILURE;
   // calls that return without stepping
   if (m->interp_ready && itask != STS_ONE_STEP && m->t >= tout)
   {
@@ -2151,17 +2192,8 @@ extern "C" int STS_ARKodeEvolve(void* mem, double tout, N_Vector yout, double* t
   // start every evolve from a clean reduction workspace (a failed launch could leave it dirty)
   cudaMemsetAsync(m->ctx->d_work, 0, sizeof(RedWork), st);
   const double clip = m->tstopset ? m->tstop : INFINITY;
-  if (!adopt_problem(m)) return STS_ERR_FAILURE;
   int ret;
-  if (fused(m))
-  {
-    if (!m->yb[0])
-    {
-      if (m->mixed && ((STS_Problem)m->user_data)->kind == STS_PROBLEM_PERIODIC) return STS_ILL_INPUT;
-      if (alloc_fused(m, NVD(m->g_y))) return STS_ERR_FAILURE;
-    }
-    ret = evolve_fused(m, tout, clip, itask);
-  }
+  if (fused(m)) ret = evolve_fused(m, tout, clip, itask);
   else ret = evolve_generic(m, tout, clip, itask);
   double tr = m->t;
   bool interp = false;
@@ -2187,12 +2219,12 @@ extern "C" int STS_ARKodeReset(void* mem, double t, N_Vector y)
   LSRKMem* m = MEM(mem);
   if (!y || NVL(y) != m->n) return STS_ILL_INPUT;
   ctx_activate(m->ctx);
+  if (m->initialized && !adopt_problem(m)) return STS_ERR_FAILURE;
   m->t            = t;
   m->tretlast     = t;
   m->interp_ready = false;
-  if (fused(m) && m->yb[0])
+  if (m->state_fused)
   {
-    if (refit_f32(m)) return STS_ERR_FAILURE;
     if (!STS_CUDA_OK(cudaMemcpyAsync(m->yb[m->par], NVD(y), m->n * sizeof(double), cudaMemcpyDeviceToDevice,
                                      m->ctx->stream)))
       return STS_ERR_FAILURE;
@@ -2224,7 +2256,7 @@ extern "C" int STS_LSRKStepTimeStageKernel(void* mem, int nlaunch, double* ms_pe
   STS_Problem p   = (STS_Problem)m->user_data;
   cudaStream_t st = m->ctx->stream;
   // (the problem may have changed since the last step, or the step lie in a checkpoint)
-  if (!m->yb[0] || ensure_stage_buffers(m) || ensure_par(m)) return STS_ERR_FAILURE;
+  if (!adopt_problem(m) || ensure_stage_buffers(m) || ensure_par(m)) return STS_ERR_FAILURE;
   if (m->mixed && !m->tuned) autotune_stage32(m, p);
   const int j     = m->last_s / 2 > 2 ? m->last_s / 2 : 2;
   cudaEvent_t e0, e1;
@@ -2449,8 +2481,8 @@ extern "C" int STS_LSRKStepWriteCheckpoint(void* mem, const char* path)
   if (!path) return STS_ILL_INPUT;
   ctx_activate(m->ctx);
   cudaStream_t st = m->ctx->stream;
-  const bool fz   = fused(m) && m->yb[0] != nullptr;
-  if ((fz && refit_f32(m)) || !STS_CUDA_OK(cudaStreamSynchronize(st))) return STS_ERR_FAILURE;
+  if ((m->initialized && !adopt_problem(m)) || !STS_CUDA_OK(cudaStreamSynchronize(st))) return STS_ERR_FAILURE;
+  const bool fz = m->state_fused;
   CkptHeader h;
   memset(&h, 0, sizeof(h));
   memcpy(h.magic, CKPT_MAGIC, 8);
@@ -2531,7 +2563,7 @@ extern "C" int STS_LSRKStepReadCheckpoint(void* mem, const char* path)
     sts_set_error("STS_LSRKStepReadCheckpoint: checkpoint written by the %s path", h.fused_path ? "fused" : "generic");
     return STS_ILL_INPUT;
   }
-  if (fz && (m->yb[0] ? refit_f32(m) : alloc_fused(m, NVD(m->g_y))))
+  if (!adopt_problem(m))
   {
     fclose(f);
     return STS_ERR_FAILURE;

@@ -125,3 +125,57 @@ def test_periodic_problem_of_another_shape(ctx, mixed):
     switch(I, B)
     I.reset(0.0, y1)
     assert np.array_equal(run(I, B, 3 * H), run(integrator(ctx, B, y1, mixed), B, 3 * H))
+
+
+# the periodic problem keeps its state elsewhere than the Dirichlet ones; 105 columns need padding
+ORDERS = [(sts.PERIODIC, (105, 80), sts.MANUFACTURED, (105, 80)), (sts.MANUFACTURED, (105, 80), sts.PERIODIC, (84, 100)),
+          (sts.PERIODIC, (84, 100), sts.UNFORCED, (105, 80))]
+
+
+@pytest.mark.parametrize("mixed", [False, True])
+@pytest.mark.parametrize("order", ORDERS, ids=str)
+def test_between_periodic_and_dirichlet(ctx, tmp_path, order, mixed):
+    A, B = make(ctx, order[0], *order[1]), make(ctx, order[2], *order[3])
+    I = integrator(ctx, A, state(ctx, A), mixed)
+    ya = run(I, A, 2 * H)
+    y1 = state(ctx, B, 2)
+    switch(I, B)
+    I.reset(0.0, y1)
+    J = integrator(ctx, B, y1, mixed)
+    assert np.array_equal(run(I, B, 2 * H), run(J, B, 2 * H))
+    I.write_checkpoint(str(tmp_path / "i"))
+    K = integrator(ctx, B, state(ctx, B, 3), mixed)
+    K.read_checkpoint(str(tmp_path / "i"))
+    assert np.array_equal(run(K, B, 4 * H), run(J, B, 4 * H))
+    switch(I, A)
+    I.reset(0.0, state(ctx, A))
+    assert np.array_equal(run(I, A, 2 * H), ya)
+    switch(I, B)
+    I.read_checkpoint(str(tmp_path / "i"))
+    assert np.array_equal(run(I, B, 4 * H), run(integrator_from(ctx, B, tmp_path / "i", mixed), B, 4 * H))
+
+
+def integrator_from(ctx, P, path, mixed):
+    I = integrator(ctx, P, state(ctx, P, 3), mixed)
+    I.read_checkpoint(str(path))
+    return I
+
+
+@pytest.mark.parametrize("mixed", [False, True])
+@pytest.mark.parametrize("order", ORDERS, ids=str)
+def test_the_state_goes_along(ctx, order, mixed):
+    """Without a reset the new problem goes on from y_n: its dense output of the last step is the old
+    one's, and back at the old problem the run continues as if it had not been left."""
+    A, B = make(ctx, order[0], *order[1]), make(ctx, order[2], *order[3])
+    I, J = (integrator(ctx, A, state(ctx, A), mixed) for _ in range(2))
+    y = A.vector()
+    for K in (I, J):
+        K.evolve(2.5 * H, y)  # dense output within the third step
+    mid = y.numpy()
+    switch(I, B)
+    yb = B.vector()
+    assert I.evolve(2.5 * H, yb)[0] == 2.5 * H and np.array_equal(yb.numpy(), mid)
+    switch(I, A)
+    assert np.array_equal(run(I, A, 6 * H), run(J, A, 6 * H))
+    switch(I, B)
+    assert np.isfinite(run(I, B, 9 * H)).all()
