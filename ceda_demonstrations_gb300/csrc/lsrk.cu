@@ -601,10 +601,16 @@ static void alloc_generic(LSRKMem* m)
 // - The state is in yb / Fb (fused path) or in g_y / g_Fn (generic path): it moves where the problem's
 //   path keeps it, with y_old of the last step (these methods' dense output needs no F).
 // - The FP32 buffers get the grid's pitch.
+// A problem of another number of points is refused: the fused kernels take their ranges from it.
 static bool adopt_problem(LSRKMem* m)
 {
   const STS_Problem p = (STS_Problem)m->user_data;
   if (m->rhs != STS_Diffusion || !p) return true;
+  if (p->nx * p->ny != m->n && !m->ssp && (fused(m) || m->initialized))
+  { // (elsewhere the RHS itself refuses it)
+    sts_set_error("LSRKStep: the problem has %lld points, the state %lld", p->nx * p->ny, m->n);
+    return false;
+  }
   cudaStream_t st = m->ctx->stream;
   if (m->kept_for != p->serial)
   {

@@ -179,3 +179,30 @@ def test_the_state_goes_along(ctx, order, mixed):
     assert np.array_equal(run(I, A, 6 * H), run(J, A, 6 * H))
     switch(I, B)
     assert np.isfinite(run(I, B, 9 * H)).all()
+
+
+@pytest.mark.parametrize("mixed", [False, True])
+@pytest.mark.parametrize("kind", [sts.MANUFACTURED, sts.PERIODIC])
+def test_another_number_of_points_is_refused(ctx, tmp_path, kind, mixed):
+    """A problem larger or smaller than the state: an error before any kernel runs, and the run goes on
+    with the right problem as if nothing had been asked."""
+    A = make(ctx, kind, 105, 80)
+    y0 = state(ctx, A)
+    want = run(integrator(ctx, A, y0, mixed), A, 4 * H)
+    I = integrator(ctx, A, y0, mixed)
+    run(I, A, 2 * H)
+    y = A.vector()
+    for other in ((105, 81), (104, 80), (210, 160)):
+        for k in (sts.MANUFACTURED, sts.PERIODIC):
+            B = make(ctx, k, *other)
+            switch(I, B)
+            for call in (lambda: I.evolve(4 * H, y), lambda: I.reset(0.0, y0),
+                         lambda: I.write_checkpoint(str(tmp_path / "c"))):
+                with pytest.raises(sts.STSError):
+                    call()
+    switch(I, A)
+    assert np.array_equal(run(I, A, 4 * H), want)
+    B = make(ctx, kind, 104, 80)
+    F = sts.LSRKStep(ctx, A, 0.0, state(ctx, B), mixed=mixed)  # from the start
+    with pytest.raises(sts.STSError):
+        F.evolve(H, B.vector())
