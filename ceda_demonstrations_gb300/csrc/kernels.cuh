@@ -424,7 +424,8 @@ __global__ void __launch_bounds__(256) stepend_kernel(ProbDev P, const StepArgs*
     up  = cur;
     cur = dn;
   }
-  xsum_block_finish<256>(acc, flags, w, slot, 1, (double)(nx * ny));
+  // (SYS in the mixed form, whose stage kernels have waits to give up)
+  xsum_block_finish<256, MIXED>(acc, flags, w, slot, 1, (double)(nx * ny));
 }
 
 // WRMS with ewt(y): mode 0 -> x = a w(y), mode 1 -> x = (a - b) w(y)

@@ -1241,6 +1241,18 @@ static int choose_step(LSRKMem* m, double target, double* hout, int* sout, bool*
 // ---------------------------------------------------------------------------------------
 // fused evolve
 // ---------------------------------------------------------------------------------------
+// The error word that a kernel sets in mapped host memory when it gives up a wait: looked at with each
+// step's result (the mixed step end orders the two), before the step is accepted, and again after the
+// synchronisation that ends every evolve.
+static bool error_word_set(LSRKMem* m)
+{
+  const int ew = *(volatile int*)m->ctx->h_err;
+  if (!ew) return false;
+  *m->ctx->h_err = 0;
+  sts_set_error("LSRKStep: %s in a stage kernel", sts_err_word_text(ew));
+  return true;
+}
+
 // Step loop of ARKodeEvolve: NORMAL mode steps until t >= tout, ONE_STEP mode takes one step;
 // steps are clipped only at `clip` (the stop time, or +inf), which they then end on exactly.
 static int evolve_fused(LSRKMem* m, double tout, double clip, int itask)
@@ -1305,12 +1317,7 @@ static int evolve_fused(LSRKMem* m, double tout, double clip, int itask)
       m->interp_ready = false; // the attempt wrote y_{n+1} over the other parity buffer
       double dsm;
       if (!slot_wait(m->ctx, SLOT_DSM, &dsm)) return STS_ERR_FAILURE;
-      if (const int ew = *(volatile int*)m->ctx->h_err)
-      {
-        *m->ctx->h_err = 0;
-        sts_set_error("LSRKStep: %s in a stage kernel", sts_err_word_text(ew));
-        return STS_ERR_FAILURE;
-      }
+      if (error_word_set(m)) return STS_ERR_FAILURE;
       m->nfe += s;
       m->stages_total += s;
       if (s > m->stage_max) m->stage_max = s;
@@ -2172,7 +2179,7 @@ extern "C" int STS_ARKodeEvolve(void* mem, double tout, N_Vector yout, double* t
   ctx_activate(m->ctx);
   cudaStream_t st = m->ctx->stream;
   auto finish     = [&](int ret, double tr) {
-    if (!STS_CUDA_OK(cudaStreamSynchronize(st))) return (int)STS_ERR_FAILURE;
+    if (!STS_CUDA_OK(cudaStreamSynchronize(st)) || error_word_set(m)) return (int)STS_ERR_FAILURE;
     if (tret) *tret = tr;
     m->tretlast = tr;
     return ret;
