@@ -364,7 +364,7 @@ struct LinSol {
   void* P_data      = nullptr;
   STS_PSolveFn psolve = nullptr;
   N_Vector r = nullptr, pv = nullptr, z = nullptr, Ap = nullptr;
-  double* d_s = nullptr; // PCG, on the device: r.z of even and odd iterations, p.(A p)
+  N_Vector sc = nullptr; // PCG, on the device: r.z of even and odd iterations, p.(A p)
   // SPGMR: Krylov basis V[0..maxl], restarts, Gram-Schmidt variant, Hessenberg + Givens;
   // SPFGMR also keeps the preconditioned basis Z[0..maxl-1]
   std::vector<N_Vector> V, Z;
@@ -383,7 +383,7 @@ static LinSol* linsol_new(int kind, N_Vector y, int pretype, int maxl, STS_Conte
   }
   LinSol* L  = new LinSol();
   L->kind    = kind;
-  L->ctx     = ctx;
+  L->ctx     = y->sunctx; // the stream of the vectors' own operations, whichever context is passed
   L->pretype = pretype;
   L->maxl    = maxl > 0 ? maxl : 5;
   L->r       = N_VClone_Sts(y);
@@ -392,7 +392,8 @@ static LinSol* linsol_new(int kind, N_Vector y, int pretype, int maxl, STS_Conte
   if (kind == LS_PCG)
   {
     L->pv = N_VClone_Sts(y);
-    if (!STS_CUDA_OK(cudaMalloc(&L->d_s, 4 * sizeof(double))))
+    L->sc = N_VNew_Sts(4, L->ctx);
+    if (!L->sc)
     {
       STS_SUNLinSolFree(L);
       return nullptr;
@@ -517,8 +518,8 @@ static int pcg_solve(LinSol* L, N_Vector x, N_Vector b, double delta)
   STS_Context ctx   = L->ctx;
   const long long n = NVL(b);
   cudaStream_t st   = ctx->stream;
-  double* const rz[2] = {L->d_s, L->d_s + 1};
-  double* const pq    = L->d_s + 2;
+  double* const rz[2] = {NVD(L->sc), NVD(L->sc) + 1};
+  double* const pq    = NVD(L->sc) + 2;
   const int g         = red_blocks(ctx, n);
   auto dot_to = [&](N_Vector u, N_Vector v, double* dst) {
     xred_kernel<0><<<g, 256, 0, st>>>(n, NVD(u), NVD(v), ctx->d_work, dst);
@@ -727,11 +728,7 @@ extern "C" int STS_SUNLinSolFree(void* LS)
   N_VDestroy_Sts(L->z);
   N_VDestroy_Sts(L->Ap);
   if (L->pv) N_VDestroy_Sts(L->pv);
-  if (L->d_s)
-  {
-    ctx_activate(L->ctx);
-    cudaFree(L->d_s);
-  }
+  if (L->sc) N_VDestroy_Sts(L->sc);
   for (N_Vector v : L->V) N_VDestroy_Sts(v);
   for (N_Vector v : L->Z) N_VDestroy_Sts(v);
   delete L;
