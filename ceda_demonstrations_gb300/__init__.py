@@ -617,6 +617,8 @@ class LSRKStep:
             _err("STS_LSRKStepReadCheckpoint")
 
     def stage_kernel_info(self):
+        """The single-stage kernel's configuration, its autotuned milliseconds per launch (0: not
+        timed) and the name of what runs."""
         v, ms = C.c_int(), C.c_double()
         buf = C.create_string_buffer(64)
         lib().STS_LSRKStepGetStageKernelInfo(self.mem, C.byref(v), C.byref(ms), buf, 64)
@@ -624,7 +626,7 @@ class LSRKStep:
 
     def stage_fusion_info(self):
         """Stages per launch in use (1: one launch per stage), the tile configuration (0: none)
-        and its rows, and the autotuner's milliseconds per launch of a group."""
+        and its rows, and the autotuner's milliseconds per launch of a group (0: not timed)."""
         ks, cfg, rows, ms = C.c_int(), C.c_int(), C.c_int(), C.c_double()
         lib().STS_LSRKStepGetStageFusion(self.mem, C.byref(ks), C.byref(cfg), C.byref(rows), C.byref(ms))
         return {"ks": ks.value, "config": cfg.value, "tile_rows": rows.value, "ms": ms.value}

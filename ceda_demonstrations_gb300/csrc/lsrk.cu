@@ -764,6 +764,10 @@ static void autotune_stage32(LSRKMem* m, STS_Problem p)
   m->fuse_ks     = 1;
   m->fuse_ti     = -1;
   m->deep_ti     = -1;
+  // times of an earlier choice (for another setting or problem) are not reported for this one
+  std::fill(std::begin(m->tune_ms), std::end(m->tune_ms), 0.0);
+  std::fill(std::begin(m->fuse_ms), std::end(m->fuse_ms), 0.0);
+  m->deep_ms = 0.0;
   if (m->stage_variant != 0 || !m->tma.ok) return;
   const bool by_default = m->fuse_req == 0 && m->fuse_tile_req < 0 && m->tma.fz_ok && m->smax >= 9;
   if (by_default && m->n < 10240LL * m->ctx->num_sms)

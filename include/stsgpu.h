@@ -248,20 +248,22 @@ int STS_LSRKStepSetMixedPrecision(void* mem, int on);
  * mbarrier pipelined tile configurations (rows per tile, ring depth, CTAs per SM) and the register-marching kernel (default), 1 = register-marching kernel,
  * 2 + k = TMA configuration k (k < 6). All variants give identical bits. */
 int STS_LSRKStepSetStageKernel(void* mem, int variant);
-/* new: the autotuner's choice (-1 = register-marching), its time per launch and its name */
+/* new: the autotuner's choice (-1 = register-marching), its time per launch and its name. The time is 0 where
+ * the choice was not timed: by default single stages are the rest of a step at most and take a fixed
+ * configuration (STS_LSRKStepTimeStageKernel times what runs) */
 int STS_LSRKStepGetStageKernelInfo(void* mem, int* variant, double* ms_per_launch, char* name,
                                    int namelen);
 /* new: mixed form, several stages per launch (temporal blocking on 120-column tiles in shared
-   memory, the same bits as one launch per stage). ks: 0 = autotuned (default: eight or four
-   stages per launch when the autotuner times that faster than one; eight, untimed, below 1.6
-   million points), 1 = off, 2..4 = that many;
+   memory, the same bits as one launch per stage). ks: 0 = by size (default: below 1.6
+   million points eight by rule, untimed; above, eight where the autotuner times them 3 % faster
+   per stage than four, else four), 1 = off, 2..4 = that many;
    config: 0 = autotuned, 1..6 = tile configuration (1: 120 x 32, three CTAs per SM; 2, 3, 5: 120 x 64,
    120 x 60 and 120 x 58, two CTAs of 256 threads per SM; 4: 120 x 64, two CTAs of 384 threads;
    6: 120 x 64, one CTA of 256 threads per SM with two tile buffers).
    Applies with the autotuned stage kernel (STS_LSRKStepSetStageKernel variant 0). */
 int STS_LSRKStepSetStageFusion(void* mem, int ks, int config);
 /* new: the stages per launch in use (1: none), the tile configuration (0: none; above 6: the
-   112-column tiles of the eight-stage groups) and its rows, and the autotuner's time per launch */
+   112-column tiles of the eight-stage groups) and its rows, and the autotuner's time per launch (0: not timed) */
 int STS_LSRKStepGetStageFusion(void* mem, int* ks, int* config, int* tile_rows, double* ms_per_launch);
 /* new: capture the fixed-s stage loop of the fused path in CUDA graphs (default on) */
 int STS_LSRKStepSetUseGraphs(void* mem, int on);
