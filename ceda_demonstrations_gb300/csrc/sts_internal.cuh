@@ -137,11 +137,6 @@ void sts_hermite(STS_Context ctx, long long n, int deg, double tau, double h, co
 // device-side reduction helpers
 // ---------------------------------------------------------------------------------------
 #ifdef __CUDACC__
-__device__ __forceinline__ long long shfl_xor_ll(long long v, int m)
-{
-  return (long long)__shfl_xor_sync(0xffffffffu, (unsigned long long)v, m);
-}
-
 // 64-bit sum over the lanes of a full warp, on the integer reduction instruction: 24-bit
 // digits (32 of them fit 29 bits), the highest one signed.
 __device__ __forceinline__ long long warp_sum_ll(long long v)
