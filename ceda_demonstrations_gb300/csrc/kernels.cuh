@@ -330,7 +330,8 @@ static __global__ void __launch_bounds__(256) stage1_32_kernel(long long n, cons
 //
 // Bound by the FP64 pipe: in the mixed form 21 FP64 instructions per point, of which the four
 // products, the neighbour sums and the conversions between the formats (which take the FP64 pipe
-// too) are integer code here (soft64.cuh), about 11 are left: 2.9 -> 2.1 ms at 8192^2 forced. On
+// too) are integer code here (soft64.cuh), about 11 are left (16.4 executed at 6144^2: warps with an
+// operand outside the integer forms' ranges take both): 2.9 -> 2.1 ms at 8192^2 forced. On
 // small grids the rows of a thread and the reduction's tail set the time (launch_stepend).
 // ---------------------------------------------------------------------------------------
 template <int RY, bool MIXED, bool FORCED>

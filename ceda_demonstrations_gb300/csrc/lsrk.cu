@@ -752,11 +752,15 @@ static void launch_stage32_idx(LSRKMem* m, STS_Problem p, const StageArgs* A, in
   launch_stage32_idx(m, p, A, im1, im2, par, iout, v);
 }
 
-// Autotuner for the mixed stage kernel: times configurations on the integrator's own buffers (a
-// realistic stage, CUDA events on the context stream, one warm and two timed launches each) and
-// keeps the fastest for this problem: by default the four-stage and eight-stage groups' large
-// tiles (on large grids; a rule picks them on small ones), with a group size or configuration
-// asked for all that match, with groups off every single-stage configuration.
+// Choice of the mixed stage kernel for this problem.
+// - By default groups. On small grids a rule picks the tiles of eight stages, untimed. On large ones
+//   one configuration of four stages and two of eight are timed, and eight are taken where they are
+//   3 % faster per stage; one launch per stage (2.6 times slower at 8192^2) is not tried.
+// - With groups off the fastest single-stage configuration; with a group size or a tile configuration
+//   asked for the fastest that matches (a configuration without a size: four stages where they are
+//   faster than one).
+// Timed on the integrator's own buffers (a realistic stage, CUDA events on the context stream, one
+// warm and two timed launches each).
 static void autotune_stage32(LSRKMem* m, STS_Problem p)
 {
   m->tuned       = true;
@@ -771,11 +775,14 @@ static void autotune_stage32(LSRKMem* m, STS_Problem p)
   if (m->stage_variant != 0 || !m->tma.ok) return;
   const bool by_default = m->fuse_req == 0 && m->fuse_tile_req < 0 && m->tma.fz_ok && m->smax >= 9;
   if (by_default && m->n < 10240LL * m->ctx->num_sms)
-  { // Grids below 1.6 million points: a launch is a chain of load, stages and barriers, and the
-    // shortest chain is the shortest tile that fits one wave (us per eight-stage launch with 16 /
-    // 32 / 48 rows: 128^2 8.3 / 10.4 / 10.7, 512^2 10.8 / 10.4 / 11.2, 1024 x 1500 25 / 22 / 23;
-    // per stage 1.0-2.8, four stages per launch 1.8-3.1). Timing all configurations costs 1.1 ms,
-    // as much as several steps on such a grid.
+  { // Grids below 1.6 million points: a launch is a chain of load, stages and barriers. 16 rows where
+    // every tile gets an SM of its own, 48 rows beyond a wave and a tenth of 32 rows (456 slots), 32
+    // between. us per eight-stage launch with 16 / 32 / 48 rows: 128^2 8.3 / 10.4 / 10.7, 512^2 10.8 /
+    // 10.4 / 11.2, 1021 x 1440 (450 tiles of 32 rows, 300 of 48) 22.6 / 18.4 / 16.4, seven grids of 460
+    // to 530 tiles of 32 rows 24.6 to 28.7 / 22.5 / 22.6 (both heights take a second wave there, so it
+    // matters little where in that range the line lies), 340 x 4570 (572) 30.7 / 28.2 / 24.6. Per
+    // stage 1.0-2.8, four stages per launch 1.8-3.1. Timing all configurations costs 1.1 ms, as much
+    // as several steps on such a grid.
     const long long sms = m->ctx->num_sms, cols = (p->nx + 111) / 112;
     m->deep_ti     = cols * ((p->ny + 15) / 16) <= sms ? 8 : cols * ((p->ny + 31) / 32) <= 3 * sms * 11 / 10 ? 7 : 6;
     m->fuse_ks     = 4;

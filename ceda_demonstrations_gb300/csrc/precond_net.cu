@@ -1607,7 +1607,6 @@ static void free_levels(STS_Net nt)
   nt->cap = 0;
 }
 
-// activation buffers for `pix` level-0 pixels (a batch of images of one size)
 // what a backward pass needs: room for the weight-gradient CTAs' sums (22 MB), the side stream
 static int wgrad_blocks(STS_Net nt);
 static bool ensure_backward(STS_Net nt)
@@ -1620,6 +1619,7 @@ static bool ensure_backward(STS_Net nt)
   return ok;
 }
 
+// activation buffers for `pix` level-0 pixels (a batch of images of one size)
 static bool ensure_capacity(STS_Net nt, long long pix)
 {
   if (pix <= nt->cap) return true;

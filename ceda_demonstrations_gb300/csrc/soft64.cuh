@@ -9,8 +9,9 @@
 // remain. Where they report true the result is the correctly rounded one, bit for bit; operands
 // outside the ranges that each one names (zeros, subnormal numbers, infinities, NaN, results
 // near the ends of the exponent range, sums with cancellation) report false, the value is then
-// meaningless, and the caller evaluates the expression with the hardware's instructions. They
-// have no branches, so that a kernel evaluates a whole point with them and tests one flag.
+// meaningless, and the caller (s64_add, s64_mul, ... below) branches to the hardware's instruction,
+// operation by operation: where the ranges hold in a whole warp no FP64 instruction is issued, a
+// predicated one would still take its slot of the pipe.
 #pragma once
 #include <cstdint>
 #include <cstring>

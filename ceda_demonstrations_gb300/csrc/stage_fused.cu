@@ -39,17 +39,20 @@ namespace {
 // per component), so a group gives the bits of KS single launches. A warp takes its rows from
 // north to south and carries the difference of neighbouring rows from one to the next; the
 // horizontal differences are scalar instructions, each taken once for the two columns that share
-// it: about 11 instructions per point and stage instead of 18 (unaligned column pairs cost moves).
+// it (unaligned column pairs cost moves). Thread instructions at 6144^2, eight stages per launch: 14
+// per evaluated point, 18.3 per DOF-stage (1.31 points are evaluated for one that is kept); four per
+// launch 15 and 17.0 (18.0 with every difference taken anew).
 //
 // HBM traffic per point and group: 12 B read (d_{j-1}, d_{j-2}, F_0; the halo overlap of
 // neighbouring tiles is mostly served by L2) + 8 B written, 20 / KS B per DOF-stage against
 // 16 B for a single-stage launch. Measured at 8192^2, us per stage: 70 for four stages per launch
-// with 18 instructions, 66 with 11, 63 for eight stages per launch; small grids, where a launch is
-// a chain of tile load, stages and barriers: 512^2 1.9 (four), 1.3 (eight); 128^2 1.8, 1.0. What
-// bounds a large launch is the chain of shared-memory loads, shuffles and barriers within a tile
-// at 16 warps per SM, not the DRAM rate (0.39 of the copy peak with eight stages) and not the
-// FP32 pipe: stage scalars from the constant bank, scalar instead of paired multiply-adds and
-// more warps per tile all measured within 3 %.
+// with every difference taken anew, 66 with the shared ones, 64 for eight stages per launch; small
+// grids, where a launch is a chain of tile load, stages and barriers: 512^2 1.9 (four), 1.3 (eight);
+// 128^2 1.8, 1.0. What bounds a large launch is the shared-memory data pipe: a warp's row takes three
+// loads and a store of 512 bytes and two shuffles there. It is busy for 80 % of an eight-stage launch
+// at 6144^2 (70 % of a four-stage one), the rest are tile loads and barriers at 16 warps per SM;
+// issue slots 49 %, FP32 pipe 50 %, DRAM 33 % (0.39 of the copy peak). Stage scalars from the
+// constant bank, scalar instead of paired multiply-adds and more warps per tile all measured within 3 %.
 // ---------------------------------------------------------------------------------------
 constexpr int FW  = 128;    // loaded tile width (floats): 32 lanes x 4 columns
 // TH output rows per tile, NT threads per CTA, MINB CTAs per SM, NSET tile buffers per CTA
