@@ -851,6 +851,7 @@ extern "C" int STS_ImplicitSolveLS(STS_Problem p, double gamma, void* LS, int pr
   else if (prec == 2) STS_SUNLinSolSetPreconditioner(L, P_data, psolve);
   else STS_SUNLinSolSetPreconditioner(L, nullptr, nullptr);
   const int rc = STS_SUNLinSolSolve(L, x, b, tol);
+  STS_ContextSynchronize(L->ctx); // x is there for every stream (a GMRES cycle ends with the update of x)
   if (iters) *iters = STS_SUNLinSolNumIters(L);
   if (relres) *relres = STS_SUNLinSolResNorm(L);
   STS_SUNLinSolSetATimes(L, nullptr, nullptr);
